@@ -1182,7 +1182,7 @@ vh_status vh_frame_stats_get(vh_volume* v, vh_frame_stats* stats, void* stream) 
   if (st != VH_OK) return st;
   stats->visible_blocks = v->h_counters->visible_count;
   stats->new_blocks = v->h_counters->new_blocks;
-  stats->active_voxels = v->h_counters->active_voxels;
+  stats->active_voxels = static_cast<uint64_t>(v->h_counters->active_voxels) + v->h_counters->literal_voxels;
   stats->updated_voxels = v->h_counters->integrated_voxels;
   stats->total_blocks = block_total(v);
   stats->observed_voxels = v->h_counters->observed_voxels;
@@ -1203,7 +1203,7 @@ vh_status vh_frame_stats_decode(const vh_volume* v, const void* counters64, vh_f
   std::memcpy(&c, counters64, sizeof(c));
   stats->visible_blocks = c.visible_count;
   stats->new_blocks = c.new_blocks;
-  stats->active_voxels = c.active_voxels;
+  stats->active_voxels = static_cast<uint64_t>(c.active_voxels) + c.literal_voxels;
   stats->updated_voxels = c.integrated_voxels;
   stats->total_blocks = std::min<uint64_t>(c.num_blocks, v->dev.max_blocks);
   stats->observed_voxels = c.observed_voxels;

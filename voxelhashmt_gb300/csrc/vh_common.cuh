@@ -40,9 +40,11 @@ struct Counters {
   unsigned long long observed_voxels;  // voxels with any layer weight > 0
   uint32_t new_blocks;         // blocks allocated by the current frame
   uint32_t integrated_voxels;  // voxel layer updates applied by the current frame
-  uint32_t active_voxels;      // voxels of the current frame that reached the layer update stage
-  uint32_t update_queue;       // next chunk of the fused layer update (a device work queue; reset per frame)
-  uint32_t pad[6];
+  uint32_t active_voxels;      // voxels of the current frame that reached the layer update stage (plain form: those
+                               // at the front of the active list)
+  uint32_t update_queue;       // next chunk of the layer update (a device work queue; reset per frame)
+  uint32_t literal_voxels;     // plain form: the rest of them, at the back of the active list
+  uint32_t pad[5];
 };
 static_assert(sizeof(Counters) == 64, "Counters is read back as one 64-byte copy");
 
@@ -60,7 +62,8 @@ static_assert(sizeof(Counters) == 64, "Counters is read back as one 64-byte copy
 //   visible_keys int4[capacity]         per visible entry {x, y, z, pool index}: written after the allocation
 //                                       by the normal-map pass, read once per chunk by the fused update
 //   active      u32[max_blocks * 512]   (block << 9 | voxel) of the current frame's voxels that pass the
-//                                       projection / depth / truncation tests (unordered)
+//                                       projection / depth / truncation tests (unordered): from the front the ones
+//                                       whose normal takes the shared samples, from the back the literal ones
 struct Volume {
   unsigned long long* slot_keys;
   uint32_t* slot_block;
@@ -178,11 +181,14 @@ __device__ __forceinline__ f3 backproject(float u, float v, float d, const Param
 //   y = 2^(k/32) * (1 + C2 r + C1 r^2 + C0 r^3) in double arithmetic (2^(j/32) from a 32-entry table),
 //   result = (float) y.
 // vh_expf returns exactly that float for every argument.  The GB300 runs FP64 at a small fraction of its FP32
-// rate, so the common path evaluates the same polynomial in float-float arithmetic (error below 2^-45.7 of
-// the result over every finite float argument) and rounds it itself; only when that value lies within 2^-40
-// of a rounding boundary (about 5 arguments in a million) does it run the double-precision sequence
-// (expf_double).  Every operation is an explicit round-to-nearest intrinsic, so the fast-math compile
-// evaluates it identically.
+// rate, so the same polynomial is evaluated in single precision and rounded here, in up to three tiers:
+//   vh_expf       arguments in [-86, 88] with only the leading terms in float-float arithmetic (error below 2^-35,
+//                 about 45 instructions, no conversions): decides unless the value lies within 2^-34 of a rounding
+//                 boundary (one argument in a thousand) or the reduced argument near a tie;
+//   vh_expf_full  float-float throughout (error below 2^-45.7 of the result over every finite float argument),
+//                 subnormal results included: decides unless within 2^-40 of a boundary (5 in a million);
+//   expf_double   the double-precision sequence.
+// Every operation is an explicit round-to-nearest intrinsic, so the fast-math compile evaluates it identically.
 namespace expf_detail {
 // bits of the double nearest 2^(j/32), minus j << 47 (so that adding k << 47 scales by 2^floor(k/32))
 static __device__ const unsigned long long kTab[32] = {
@@ -254,7 +260,7 @@ static __device__ __noinline__ float expf_double(float x) {
   return __double2float_rn(y);
 }
 
-__device__ __forceinline__ float vh_expf(float x) {
+static __device__ __noinline__ float vh_expf_full(float x) {
   using namespace expf_detail;
   if (!(x >= kLo && x <= kHi)) return expf_double(x);
   // P = x * 32/ln2 exactly, as p0 + e0 + p1 + e1 + p2 (the last product's rounding is below 2^-59)
@@ -317,6 +323,39 @@ __device__ __forceinline__ float vh_expf(float x) {
   return __uint_as_float(static_cast<uint32_t>(static_cast<int>(n)));
 }
 
+__device__ __forceinline__ float vh_expf(float x) {
+  using namespace expf_detail;
+  if (!(x >= -86.0f && x <= 88.0f)) return vh_expf_full(x);
+  // P = x * 32/ln2 = p0 + b, k = p0 rounded by adding 1.5 * 2^23 (k in the low bits of kf), r = P - k = rh + rl
+  constexpr float kRound = 0x1.8p+23f;
+  const float p0 = __fmul_rn(x, kIH);
+  const float kf = __fadd_rn(p0, kRound);
+  const float a = __fsub_rn(p0, __fsub_rn(kf, kRound));
+  const float b = __fmaf_rn(x, kIM, __fmaf_rn(x, kIH, -p0));
+  float rh, rl;
+  fast_two_sum(a, b, rh, rl);  // a is 0 or a multiple of p0's last place, which |b| does not reach
+  // q = C2 r + (C1 + C0 r) r^2: the first product in float-float, the rest (below 2^-14) in single precision
+  const float m = __fmul_rn(__fmaf_rn(kC0H, rh, kC1H), __fmul_rn(rh, rh));
+  float c, ce;
+  two_prod(kC2H, rh, c, ce);
+  const float s = __fadd_rn(__fmaf_rn(kC2M, rh, __fmaf_rn(kC2H, rl, ce)), m);
+  // Z = 2^(j/32) (1 + q), result = Z * 2^e with k = 32 e + j
+  const uint32_t kb = __float_as_uint(kf);
+  const float2 T = kTabF[kb & 31U];
+  float zh1, zl1, Zh, Zl;
+  two_prod(T.x, c, zh1, zl1);
+  zl1 = __fadd_rn(zl1, __fmaf_rn(T.x, s, __fmaf_rn(T.y, c, T.y)));
+  fast_two_sum(T.x, zh1, Zh, Zl);
+  fast_two_sum(Zh, __fadd_rn(Zl, zl1), Zh, Zl);
+  // half the spacing of the floats at Zh (a quarter below 1.0): Zh unless Z lies near a rounding boundary
+  const uint32_t zb = __float_as_uint(Zh);
+  const float half = __uint_as_float((zb & 0x7f800000U) - 0x0c000000U);
+  if (!(fabsf(rh) < 0.5f - 0x1p-20f) || !(__fsub_rn(half, fabsf(Zl)) > 0x1p-34f) || (Zh == 1.0f && Zl < -0x1p-26f)) {
+    return vh_expf_full(x);
+  }
+  return __uint_as_float(zb + ((kb & ~31U) << 18));
+}
+
 // x / 65535.0f for x in {0, 1, ..., 65535}: reciprocal multiply plus one fused correction step (Markstein's
 // method).  Equal to the IEEE quotient on all 65536 inputs (checked exhaustively on the host), at 3 instructions.
 __device__ __forceinline__ float div65535(float x) {
@@ -332,6 +371,8 @@ __device__ __forceinline__ float gaussian(float sq, float k) { return __expf(-sq
 #else
 __device__ __forceinline__ float gaussian(float sq, float k) { return vh_expf(-sq * k); }
 #endif
+// gaussian(sq, k) is exactly 0: the exponent is below log 2^-150 (false for a NaN)
+__device__ __forceinline__ bool gaussian_is_zero(float sq, float k) { return -sq * k < -0x1.9fe368p6f; }
 __device__ __forceinline__ float disc_threshold(const Params& p, float ref) {
   return fmaxf(p.disc_base, p.disc_rel * fmaxf(ref, 0.0f));
 }

@@ -96,6 +96,7 @@ __device__ __forceinline__ void bilateral_taps(const Smem& S, int tx, int ty, fl
       }
       const float w = S.spatial[(dv + kR) * (2 * kR + 1) + (du + kR)] * __expf(-e);
 #else
+      if (gaussian_is_zero(range, p.filter_k_range)) continue;  // adds zeros
       float w = S.spatial[(dv + kR) * (2 * kR + 1) + (du + kR)] * gaussian(range, p.filter_k_range);
       if (has_cn) {
         const float4 sn = S.normal[ty + kR + dv][tx + kR + du];
@@ -158,6 +159,7 @@ __device__ __forceinline__ void begin_frame(Counters* counters) {
   counters->integrated_voxels = 0U;
   counters->active_voxels = 0U;
   counters->update_queue = 0U;
+  counters->literal_voxels = 0U;
 }
 
 }  // namespace filt

@@ -13,7 +13,7 @@
 // The per-voxel bilateral normal (estimateSurfaceNormalCamera, :754-832) evaluates 9 base normals, each from
 // 4 bilinear depth samples, plus 10 more samples: 50 bilinear samples per voxel, all at (u + i, v + j) for
 // integer i, j in [-2, 2].  Whenever the shifted coordinates are exact -- (u-1)+1 == u, (u+1)-1 == u and the
-// same for v, which the kernel checks -- the reference evaluates every one of those samples at the same
+// same for v, which the classify pass checks -- the reference evaluates every one of those samples at the same
 // float coordinates, so the 21 distinct samples are computed once and reused; the result is bit-identical.
 // Otherwise (u or v within 2 of a power of two, or below 1) the literal 50-sample sequence runs.
 //
@@ -127,11 +127,11 @@ __device__ __noinline__ bool base_normal_literal(const float* __restrict__ depth
 
 // estimateSurfaceNormalCamera (cuda_tsdf_integrator.cu:754-832), literal evaluation order
 __device__ __noinline__ bool surface_normal_literal(const float* __restrict__ depth, const Params& p, float u,
-                                                    float v, const float gs[3], f3& normal) {
+                                                    float v, const float gs[3], float& cd, f3& normal) {
+  const bool sampled = sample_bilinear(depth, p, u, v, cd);
   f3 cn;
   if (!base_normal_literal(depth, p, u, v, cn)) return false;
-  float cd;
-  if (!sample_bilinear(depth, p, u, v, cd)) return false;
+  if (!sampled) return false;
   const f3 cp = backproject(u, v, cd, p);
   cn = orient_toward_camera(cn, cp);
   f3 wsum = mk3(0.0f, 0.0f, 0.0f);
@@ -168,27 +168,8 @@ __device__ __noinline__ bool surface_normal_literal(const float* __restrict__ de
   return norm3(n) > 1e-6f;
 }
 
-// The 21 distinct sample positions (i, j) of the fast path, i, j in [0, 4] (offsets i-2, j-2): row 0 and row 4
-// hold columns 1..3, rows 1..3 all five columns.
-__device__ __forceinline__ void sample_position(int s, int& i, int& j) {
-  if (s < 3) {
-    j = 0;
-    i = s + 1;
-  } else if (s < 18) {
-    j = 1 + (s - 3) / 5;
-    i = (s - 3) % 5;
-  } else {
-    j = 4;
-    i = s - 17;
-  }
-}
-__device__ __forceinline__ int sample_slot(int i, int j) {
-  return j == 0 ? i - 1 : (j == 4 ? 17 + i : 3 + (j - 1) * 5 + i);
-}
-__device__ __forceinline__ float pick5(int k, float a0, float a1, float a2, float a3, float a4) {
-  return k == 0 ? a0 : (k == 1 ? a1 : (k == 2 ? a2 : (k == 3 ? a3 : a4)));
-}
-
+// The sample positions (i, j) of the fast path, i, j in [0, 4] (offsets i - 2, j - 2): row 0 and row 4 hold columns
+// 1..3, rows 1..3 all five columns, 21 in all.
 constexpr int kSamples = 21;
 
 // Per-thread scratch of the fast path: backprojected sample points, [component][sample][thread] so a warp's
@@ -200,62 +181,192 @@ struct NormalScratch {
   float z[kSamples][kT];
 };
 
+// x / b correctly rounded, inv_b = 1 / b correctly rounded: two corrections of x * inv_b by the exact remainder
+// (Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", 1990: a faithful quotient
+// corrected with a correctly rounded reciprocal is the correctly rounded one), for operands whose quotient and
+// remainder neither overflow nor underflow.
+__device__ __forceinline__ float div_known(float x, float b, float inv_b) {
+  float q = __fmul_rn(x, inv_b);
+  q = __fmaf_rn(__fmaf_rn(-q, b, x), inv_b, q);
+  return __fmaf_rn(__fmaf_rn(-q, b, x), inv_b, q);
+}
+
+// The camera of a launch: reciprocal focal lengths, and whether the intrinsics are of ordinary size (2^-20..2^20, or
+// a principal point at 0), so that for depths in 2^-20..2^20 div_known's operands are too: |u - cx| is 0 or at
+// least 2^-43.
+struct CameraDiv {
+  float inv_fx, inv_fy;
+  bool ok;
+};
+__device__ __forceinline__ CameraDiv camera_div(const Params& p) {
+  auto ordinary = [](float a) { return fabsf(a) >= 0x1p-20f && fabsf(a) <= 0x1p20f; };
+  return CameraDiv{1.0f / p.fx, 1.0f / p.fy,
+                   ordinary(p.fx) && ordinary(p.fy) && (p.cx == 0.0f || ordinary(p.cx)) &&
+                       (p.cy == 0.0f || ordinary(p.cy)) && p.width <= (1 << 20) && p.height <= (1 << 20)};
+}
+
+// orient_unit_toward_camera out of line (normals almost perpendicular to the ray)
+__device__ __noinline__ f3 orient_unit_exact(f3 n, f3 pc) { return orient_unit_toward_camera(n, pc); }
+
+// sampleDepthBilinear across a depth discontinuity: the taps within thr of the nearest one; d when they carry no weight
+__device__ __noinline__ float bilinear_gated(float d00, float d10, float d01, float d11, float ref, float thr, float tx,
+                                             float ty) {
+  const float w00 = (1.0f - tx) * (1.0f - ty), w10 = tx * (1.0f - ty), w01 = (1.0f - tx) * ty, w11 = tx * ty;
+  float wds = 0.0f, ws = 0.0f;
+  if (!(fabsf(d00 - ref) > thr)) {
+    wds += w00 * d00;
+    ws += w00;
+  }
+  if (!(fabsf(d10 - ref) > thr)) {
+    wds += w10 * d10;
+    ws += w10;
+  }
+  if (!(fabsf(d01 - ref) > thr)) {
+    wds += w01 * d01;
+    ws += w01;
+  }
+  if (!(fabsf(d11 - ref) > thr)) {
+    wds += w11 * d11;
+    ws += w11;
+  }
+  return ws > 1e-6f ? wds / ws : ref;
+}
+
 // estimateSurfaceNormalCamera through the 21 distinct samples, valid when the shifted coordinates are exact
-// (checked by the caller).  Rolled loops keep the code small; the samples live in shared memory.
+// (checked by the caller).
+//
+// The kernel is bound by instruction issue, so this is written for few instructions with the same results:
+//   - The samples share a window of 6x6 pixels (32 of them read, not 84): sample (i, j) lies between window columns
+//     i, i + 1 and rows j, j + 1, its fractions depend on the column and the row alone, and a row's horizontal
+//     interpolation serves the samples above and below it.  Columns and rows outside the image are clamped, as the
+//     reference clamps a sample's second tap, and the samples outside it are marked invalid.  Where the reference
+//     falls back to the nearest depth, that is one of the sample's four taps.
+//   - Divisions by the focal lengths multiply by their reciprocals and correct (div_known).
+//   - A neighbour whose range weight is exactly 0 adds nothing and is left out before its normal is computed.
+//   - |n| > 1e-6 of a normalised vector is known from its length before (finite, above 1e-6): no second root.
+//   - The sign of a normal's dot product with the viewing direction is the sign of its dot product with the point
+//     itself unless they are almost perpendicular: no root and no division.
+//   - The centre's own normal is used again for its own tap, whose range weight is 1.
+// Rolled loops keep the code within the instruction cache; the points live in shared memory.
 template <int kT>
-__device__ __forceinline__ bool surface_normal_fast(const float* __restrict__ depth, const Params& p, float u, float v,
-                                                    const float gs[3], NormalScratch<kT>& S, int t, f3& normal) {
+__device__ __forceinline__ bool surface_normal_fast(const float* __restrict__ depth, const Params& p,
+                                                    const CameraDiv& cd_, float u, float v, const float gs[3],
+                                                    NormalScratch<kT>& S, int t, float& d, f3& normal) {
   const float um1 = u - 1.0f, up1 = u + 1.0f, vm1 = v - 1.0f, vp1 = v + 1.0f;
-  const float U0 = um1 - 1.0f, U4 = up1 + 1.0f, V0 = vm1 - 1.0f, V4 = vp1 + 1.0f;
+  const float sx0 = um1 - 1.0f, sx4 = up1 + 1.0f;
+  const int x0 = static_cast<int>(floorf(u)) - 2, y0 = static_cast<int>(floorf(v)) - 2;
+  const float wmax = static_cast<float>(p.width - 1), hmax = static_cast<float>(p.height - 1);
   uint32_t ok = 0U;
 #pragma unroll 1
-  for (int s = 0; s < kSamples; ++s) {
-    int i, j;
-    sample_position(s, i, j);
-    const float su = pick5(i, U0, um1, u, up1, U4);
-    const float sv = pick5(j, V0, vm1, v, vp1, V4);
-    float d;
-    if (sample_bilinear(depth, p, su, sv, d)) {
-      ok |= 1U << s;
-      const f3 q = backproject(su, sv, d, p);
-      S.x[s][t] = q.x;
-      S.y[s][t] = q.y;
-      S.z[s][t] = q.z;
+  for (int j = 0; j < 5; ++j) {
+    const float sv = j == 0 ? vm1 - 1.0f : (j == 1 ? vm1 : (j == 2 ? v : (j == 3 ? vp1 : vp1 + 1.0f)));
+    const float flv = floorf(sv);
+    const float ty = sv - flv;
+    const bool lower = floorf(sv + 0.5f) != flv;
+    const bool row_in = sv >= 0.0f && sv <= hmax;
+    const float pv = sv - p.cy;
+    const bool full = j > 0 && j < 4;
+    const int i0 = full ? 0 : 1, i1 = full ? 5 : 4;
+    int s = j == 0 ? 0 : (j == 4 ? 18 : 5 * j - 2);  // sample slot of column i0
+    const float* r0 = depth + static_cast<size_t>(min(max(y0 + j, 0), p.height - 1)) * p.width;
+    const float* r1 = depth + static_cast<size_t>(min(max(y0 + j + 1, 0), p.height - 1)) * p.width;
+    int c = min(max(x0 + i0, 0), p.width - 1);
+    float d00 = __ldg(r0 + c), d01 = __ldg(r1 + c);
+#pragma unroll 1
+    for (int i = i0; i < i1; ++i, ++s) {
+      const float su = i == 0 ? sx0 : (i == 1 ? um1 : (i == 2 ? u : (i == 3 ? up1 : sx4)));
+      c = min(max(x0 + i + 1, 0), p.width - 1);
+      const float d10 = __ldg(r0 + c), d11 = __ldg(r1 + c);
+      const float flu = floorf(su);
+      const float tx = su - flu;
+      const bool right = floorf(su + 0.5f) != flu;
+      const float ref = right ? (lower ? d11 : d10) : (lower ? d01 : d00);
+      const bool in = row_in && su >= 0.0f && su <= wmax && ref > 0.0f;
+      float ds = ref;
+      if (d00 > 0.0f && d10 > 0.0f && d01 > 0.0f && d11 > 0.0f) {
+        const float thr = disc_threshold(p, ref);
+        const float mn = fminf(fminf(d00, d10), fminf(d01, d11));
+        const float mx = fmaxf(fmaxf(d00, d10), fmaxf(d01, d11));
+        const float top = d00 + (d10 - d00) * tx;
+        const float bottom = d01 + (d11 - d01) * tx;
+        ds = top + (bottom - top) * ty;
+        if (!(mx - mn <= thr)) ds = bilinear_gated(d00, d10, d01, d11, ref, thr, tx, ty);
+      }
+      if (in) {
+        ok |= 1U << s;
+        const float nx = (su - p.cx) * ds, ny = pv * ds;
+        float x, y;
+        if (cd_.ok && ds >= 0x1p-20f && ds <= 0x1p20f) {
+          x = div_known(nx, p.fx, cd_.inv_fx);
+          y = div_known(ny, p.fy, cd_.inv_fy);
+        } else {
+          x = nx / p.fx;
+          y = ny / p.fy;
+        }
+        S.x[s][t] = x;
+        S.y[s][t] = y;
+        S.z[s][t] = ds;
+      }
+      d00 = d10;
+      d01 = d11;
     }
   }
-  auto point = [&](int i, int j) {
-    const int s = sample_slot(i, j);
-    return mk3(S.x[s][t], S.y[s][t], S.z[s][t]);
-  };
-  auto valid = [&](int i, int j) { return (ok >> sample_slot(i, j)) & 1U; };
-  // base normal at (i, j): estimateSurfaceNormalBaseCamera on the cached samples
-  auto base = [&](int i, int j, f3& n) -> bool {
-    if (!(valid(i - 1, j) && valid(i + 1, j) && valid(i, j - 1) && valid(i, j + 1))) return false;
-    n = normalize3(cross3(sub3(point(i, j + 1), point(i, j - 1)), sub3(point(i + 1, j), point(i - 1, j))));
-    return norm3(n) > 1e-6f;
-  };
-  f3 cn;
-  if (!base(2, 2, cn)) return false;
-  if (!valid(2, 2)) return false;
-  const f3 cp = point(2, 2);
-  const float cd = cp.z;
-  cn = orient_unit_toward_camera(cn, cp);
-  f3 wsum = mk3(0.0f, 0.0f, 0.0f);
+  constexpr int kCentre = 10;
+  constexpr uint32_t kCentreNeeds = (1U << 5) | (1U << 9) | (1U << 10) | (1U << 11) | (1U << 15);
+  d = S.z[kCentre][t];
+  if ((ok & kCentreNeeds) != kCentreNeeds) return false;
+  auto point = [&](int s) { return mk3(S.x[s][t], S.y[s][t], S.z[s][t]); };
+  const f3 cp = point(kCentre);
+  f3 cn = mk3(0.0f, 0.0f, 0.0f);
+  f3 wsum = cn;
   float ws = 0.0f;
+  // the centre's normal (k = -1), then the nine taps: one copy of the normal's and of the exponential's code
 #pragma unroll 1
-  for (int k = 0; k < 9; ++k) {
-    const int i = 1 + k % 3, j = 1 + k / 3;
-    f3 sn;
-    if (!base(i, j, sn)) continue;
-    if (!valid(i, j)) continue;
-    const f3 sp = point(i, j);
-    sn = orient_unit_toward_camera(sn, sp);
-    const float delta = sp.z - cd;
+  for (int k = -1; k < 9; ++k) {
+    const int jr = k < 0 ? 1 : k / 3;                               // sample row jr + 1
+    const int s = k < 0 ? kCentre : 4 + 5 * jr + (k - 3 * jr);      // this neighbour's sample
+    const int a = s - (jr == 0 ? 4 : 5), b = s + (jr == 2 ? 4 : 5);  // above, below
+    const uint32_t needs = (7U << (s - 1)) | (1U << a) | (1U << b);
+    if ((ok & needs) != needs) continue;
+    f3 sn = cn;
+    float range = 0.0f;
+    if (k != 4) {
+      const f3 sp = point(s);
+      const float delta = sp.z - cp.z;
+      range = delta * delta;
+      if (gaussian_is_zero(range, p.normal_k_range)) continue;
+      // estimateSurfaceNormalBaseCamera on the samples, toward the camera
+      const f3 cr = cross3(sub3(point(b), point(a)), sub3(point(s + 1), point(s - 1)));
+      const float len = norm3(cr);
+      if (!(len > 1e-6f && len <= 3.402823466e38f)) {
+        if (k < 0) return false;
+        continue;
+      }
+      sn = mul3(cr, 1.0f / len);
+      const float dot = dot3(sn, sp), mag = fabsf(sp.x) + fabsf(sp.y) + fabsf(sp.z);
+      // both dot products round to within 4 units in the last place of mag (or mag / |sp|)
+      if (fabsf(dot) > 1e-5f * mag && sp.z > 1e-5f && mag < 1e18f) {
+        if (dot > 0.0f) sn = mul3(sn, -1.0f);
+      } else {
+        sn = orient_unit_exact(sn, sp);
+      }
+      if (k < 0) {
+        cn = sn;
+        continue;
+      }
+    }
     const float cosine = clampf(dot3(cn, sn), -1.0f, 1.0f);
     const float ad = 1.0f - cosine;
-    const int r2 = (i - 2) * (i - 2) + (j - 2) * (j - 2);
-    const float w = pick5(r2, gs[0], gs[1], gs[2], 0.0f, 0.0f) * gaussian(delta * delta, p.normal_k_range) *
-                    gaussian(ad * ad, p.normal_k_angular);
+    float w = k == 4 ? gs[0] : ((k & 1) ? gs[1] : gs[2]);
+    float sq = range, kk = p.normal_k_range;
+#pragma unroll 1
+    for (int e = k == 4 ? 1 : 0; e < 2; ++e) {  // the centre's range weight is 1
+      if (e == 1) {
+        sq = ad * ad;
+        kk = p.normal_k_angular;
+      }
+      w *= gaussian(sq, kk);
+    }
     wsum.x += sn.x * w;
     wsum.y += sn.y * w;
     wsum.z += sn.z * w;
@@ -273,14 +384,12 @@ __device__ __forceinline__ bool surface_normal_fast(const float* __restrict__ de
   return norm3(n) > 1e-6f;
 }
 
-template <int kT>
-__device__ __forceinline__ bool surface_normal(const float* __restrict__ depth, const Params& p, float u, float v,
-                                               const float gs[3], NormalScratch<kT>& S, int t, f3& normal) {
+// The fast path's conditions: the shifted coordinates exact, and the farthest samples (whose last bit may round) in
+// the pixel expected.
+__device__ __forceinline__ bool shifts_exact(float u, float v) {
   const float um1 = u - 1.0f, up1 = u + 1.0f, vm1 = v - 1.0f, vp1 = v + 1.0f;
-  if (!(um1 + 1.0f == u && up1 - 1.0f == u && vm1 + 1.0f == v && vp1 - 1.0f == v)) {
-    return surface_normal_literal(depth, p, u, v, gs, normal);
-  }
-  return surface_normal_fast<kT>(depth, p, u, v, gs, S, t, normal);
+  return um1 + 1.0f == u && up1 - 1.0f == u && vm1 + 1.0f == v && vp1 - 1.0f == v &&
+         floorf(up1 + 1.0f) == floorf(u) + 2.0f && floorf(vp1 + 1.0f) == floorf(v) + 2.0f;
 }
 
 // computeObservationWeightGpu (cuda_tsdf_integrator.cu:429-450)
@@ -381,22 +490,24 @@ __device__ __forceinline__ bool integrate_sample(const Params& p, float4& L0, fl
   const float plane_offset = dot3(n, sp);
   int empty = -1, best = -1;
   float best_delta = 1e30f;
-#pragma unroll
+  f3 pn = mk3(0.0f, 0.0f, 0.0f);  // the normal of layer `best`
+#pragma unroll 1
   for (int l = 0; l < 3; ++l) {
-    const float4& L = l == 0 ? L0 : (l == 1 ? L1 : L2);
+    const float4 L = l == 0 ? L0 : (l == 1 ? L1 : L2);
     if (!layer_valid(L)) {
       if (empty < 0) empty = l;
       continue;
     }
+    // a layer farther than merge_tol is never the merged one (the best match is taken only within merge_tol)
+    const float delta = fabsf(L.y - sc);
+    if (!(delta <= p.merge_tol) || !(delta < best_delta)) continue;
     const f3 ln = unpack_normal(__float_as_uint(L.w));
     if (dot3(ln, n) < p.layer_normal_cos) continue;
-    const float delta = fabsf(L.y - sc);
-    if (delta < best_delta) {
-      best_delta = delta;
-      best = l;
-    }
+    best_delta = delta;
+    best = l;
+    pn = ln;
   }
-  const int li = (best >= 0 && best_delta <= p.merge_tol) ? best : empty;
+  const int li = best >= 0 ? best : empty;
   if (li < 0) return false;
   float4 L = li == 0 ? L0 : (li == 1 ? L1 : L2);
   const float pw = L.x;
@@ -407,7 +518,6 @@ __device__ __forceinline__ bool integrate_sample(const Params& p, float4& L0, fl
   L.y = pw > 0.0f ? ((L.y * pw + sc * ew) / nwt) : sc;
   L.z = pw > 0.0f ? ((L.z * pw + plane_offset * ew) / nwt) : plane_offset;
   if (pw > 0.0f) {
-    const f3 pn = unpack_normal(__float_as_uint(L.w));
     blended = normalize3(mul3(add3(mul3(pn, pw), mul3(n, ew)), 1.0f / nwt));
     if (norm3(blended) <= 1e-6f) blended = n;
   }
@@ -525,8 +635,7 @@ __device__ __forceinline__ bool integrate_bin16(const Params& p, const Volume& V
 
 // First part of integrateActiveBlocksKernel for one voxel (:849-877): voxel centre, projection, bilinear
 // depth, truncation test.  Returns false when the reference returns before touching the voxel.
-__device__ __forceinline__ bool voxel_prefix(const float* __restrict__ depth, const Params& p, const int4& bk, int li,
-                                             f3& pc, float& u, float& v, float& d) {
+__device__ __forceinline__ bool voxel_projection(const Params& p, const int4& bk, int li, f3& pc, float& u, float& v) {
   const int lx = li & 7, ly = (li >> 3) & 7, lz = li >> 6;
   const f3 pw = mk3((static_cast<float>(bk.x * kBlockSide + lx) + 0.5f) * p.voxel_size,
                     (static_cast<float>(bk.y * kBlockSide + ly) + 0.5f) * p.voxel_size,
@@ -536,24 +645,31 @@ __device__ __forceinline__ bool voxel_prefix(const float* __restrict__ depth, co
   if (pc.z <= 1e-6f) return false;
   u = p.fx * pc.x / pc.z + p.cx;
   v = p.fy * pc.y / pc.z + p.cy;
-  if (!(u >= 0.0f && u <= static_cast<float>(p.width - 1) && v >= 0.0f && v <= static_cast<float>(p.height - 1))) {
-    return false;
-  }
+  return u >= 0.0f && u <= static_cast<float>(p.width - 1) && v >= 0.0f && v <= static_cast<float>(p.height - 1);
+}
+
+__device__ __forceinline__ bool voxel_prefix(const float* __restrict__ depth, const Params& p, const int4& bk, int li,
+                                             f3& pc, float& u, float& v, float& d) {
+  if (!voxel_projection(p, bk, li, pc, u, v)) return false;
   if (!sample_bilinear(depth, p, u, v, d)) return false;
   return !(d - pc.z <= -p.truncation);
 }
 
-// Rest of integrateActiveBlocksKernel (:879-899): bilateral normal, observation weight, surface point,
-// direction bin.  Returns the direction bin, or -1 when the reference skips the voxel.
+// Rest of integrateActiveBlocksKernel (:879-899) for a voxel that passed voxel_prefix: bilinear depth d and bilateral
+// normal at its projection (u, v), observation weight, surface point, direction bin.  Returns the direction bin, or
+// -1 when the reference skips the voxel.
 template <int kT>
-__device__ __forceinline__ int voxel_observation(const float* __restrict__ depth, const Params& p, f3 pc, float u,
-                                                 float v, float d, const float gs[3], NormalScratch<kT>& S, int t,
-                                                 float& sc, f3& spw, f3& nw, float& obs) {
-  const float sd = d - pc.z;
+__device__ __forceinline__ int voxel_observation(const float* __restrict__ depth, const Params& p, const CameraDiv& cd,
+                                                 f3 pc, float u, float v, bool literal, const float gs[3],
+                                                 NormalScratch<kT>& S, int t, float& sc, f3& spw, f3& nw, float& obs) {
   const f3 view = normalize3(pc);
+  float d = 0.0f;
   float view_w = 1.0f;
   f3 nc = mul3(view, -1.0f);
-  if (surface_normal<kT>(depth, p, u, v, gs, S, t, nc)) view_w = fabsf(dot3(nc, view));
+  const bool have = literal ? surface_normal_literal(depth, p, u, v, gs, d, nc)
+                            : surface_normal_fast<kT>(depth, p, cd, u, v, gs, S, t, d, nc);
+  if (have) view_w = fabsf(dot3(nc, view));
+  const float sd = d - pc.z;
   obs = observation_weight(p, d, sd, view_w);
   if (obs <= 0.0f) return -1;
   spw = xform_point(p.T_wc, backproject(u, v, d, p));
@@ -565,12 +681,16 @@ __device__ __forceinline__ int voxel_observation(const float* __restrict__ depth
 }
 
 // Pass 1: every voxel of every visible block; the ones that reach the layer update in the reference are
-// appended to V.active (warp-aggregated: one atomic per warp).  Cheap and uniform per voxel.
+// appended to V.active (warp-aggregated: one atomic per warp).  Cheap and uniform per voxel.  The voxels whose
+// normal needs the literal 50-sample sequence go to the back of the list, so that the update's warps are of one
+// kind: one such lane made its whole warp run that sequence, three times the instructions, and with powers of two at
+// columns 32, 64, 128, 256 and as many rows a fifth of the warps of a 320x240 frame had one.
 __global__ void __launch_bounds__(kThreads) classify_kernel(const float* __restrict__ depth, const Volume V,
                                                             const Params p) {
   const uint32_t nvis = V.counters->visible_count;
   const unsigned long long total = static_cast<unsigned long long>(nvis) * kBlockVoxels;
   const int lane = threadIdx.x & 31;
+  const uint32_t last = V.max_blocks * static_cast<uint32_t>(kBlockVoxels) - 1U;  // max_blocks <= 2^23
   const unsigned long long stride = static_cast<unsigned long long>(gridDim.x) * blockDim.x;
   // every lane of a warp runs the same number of iterations (the total is a multiple of 512)
   for (unsigned long long i = static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
@@ -578,57 +698,99 @@ __global__ void __launch_bounds__(kThreads) classify_kernel(const float* __restr
     const uint32_t item = static_cast<uint32_t>(i >> 9);
     const int li = static_cast<int>(i & 511U);
     const uint32_t b = V.slot_block[V.visible[item]];
-    bool pass = false;
+    bool pass = false, literal = false;
     if (li == 0 && b != kInvalidBlock) V.block_stamp[b] = V.counters->frame;  // for incremental meshing
     if (b != kInvalidBlock) {
       const int4 bk = V.block_keys[b];
       f3 pc;
       float u, v, d;
       pass = voxel_prefix(depth, p, bk, li, pc, u, v, d);
+      literal = pass && !shifts_exact(u, v);
     }
-    const uint32_t ballot = __ballot_sync(0xffffffffU, pass);
+    const uint32_t ballot = __ballot_sync(0xffffffffU, pass && !literal);
+    const uint32_t lits = __ballot_sync(0xffffffffU, literal);
+    const uint32_t below = (1U << lane) - 1U;
     if (ballot) {
       uint32_t base = 0;
       if (lane == 0) base = atomicAdd(&V.counters->active_voxels, static_cast<uint32_t>(__popc(ballot)));
       base = __shfl_sync(0xffffffffU, base, 0);
-      if (pass) V.active[base + __popc(ballot & ((1U << lane) - 1U))] = (b << 9) | static_cast<uint32_t>(li);
+      if (pass && !literal) V.active[base + __popc(ballot & below)] = (b << 9) | static_cast<uint32_t>(li);
+    }
+    if (lits) {
+      uint32_t base = 0;
+      if (lane == 0) base = atomicAdd(&V.counters->literal_voxels, static_cast<uint32_t>(__popc(lits)));
+      base = __shfl_sync(0xffffffffU, base, 0);
+      if (literal) V.active[last - (base + __popc(lits & below))] = (b << 9) | static_cast<uint32_t>(li);
     }
   }
 }
 
 // Pass 2: the layer update of the active voxels, one voxel per thread, no CTA barriers: the expensive
-// bilateral normal runs only where the reference runs it, and slow voxels no longer hold a whole block.
-constexpr int kUpdateThreads = 128;
+// bilateral normal runs only where the reference runs it, and slow voxels no longer hold a whole block.  A warp
+// takes the next 32 voxels of the list from a device work queue, the literal ones first (their warps run longest).
+//
+// The kernel is bound by instruction fetch before issue: its working set of code decides.  The 21 samples, the 9
+// taps and the 3 layers are rolled loops with one copy each of the sample, the normal, the exponential and the
+// normal's unpacking; unrolled rows of samples ran 25 % fewer instructions in the same time (half of the warps waiting
+// for instructions at any moment).  28 warps per SM (72 registers, the normal scratch fills the shared memory): 1,131
+// us for a room frame of 5.4 M active voxels, 1,158 with 24 warps.  Before: 2,661 us, the literal lanes inside the
+// warps of the others, 84 depth loads a voxel and a longer exponential; 1,698 us without the separate literal list.
+constexpr int kUpdateThreads = 128, kUpdateMinB = 7;
 
-__global__ void __launch_bounds__(kUpdateThreads) update_kernel(const float* __restrict__ depth, const Volume V,
-                                                                const Params p) {
+template <bool kFp16>
+__global__ void __launch_bounds__(kUpdateThreads, kUpdateMinB) update_kernel(const float* __restrict__ depth, const Volume V,
+                                                                   const Params p) {
   __shared__ NormalScratch<kUpdateThreads> S;
-  const uint32_t n = V.counters->active_voxels;
-  const uint32_t padded = (n + 31U) & ~31U;
+  const uint32_t n = V.counters->active_voxels, n_literal = V.counters->literal_voxels;
+  const uint32_t literal_chunks = (n_literal + 31U) / 32U, chunks = literal_chunks + (n + 31U) / 32U;
+  const uint32_t last = V.max_blocks * static_cast<uint32_t>(kBlockVoxels) - 1U;
   const int lane = threadIdx.x & 31;
   const float gs[3] = {gaussian(0.0f, p.normal_k_spatial), gaussian(1.0f, p.normal_k_spatial),
                        gaussian(2.0f, p.normal_k_spatial)};
-  const uint32_t stride = gridDim.x * blockDim.x;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < padded; i += stride) {
+  const CameraDiv cam = camera_div(p);
+  uint32_t sum_updated = 0U, sum_newly = 0U;
+  uint32_t next = 0U;
+  if (lane == 0) next = atomicAdd(&V.counters->update_queue, 1U);
+  for (;;) {
+    const uint32_t chunk = __shfl_sync(0xffffffffU, next, 0);
+    if (chunk >= chunks) break;
+    if (lane == 0) next = atomicAdd(&V.counters->update_queue, 1U);  // in flight during this chunk's work
+    const bool literal = chunk < literal_chunks;
+    const uint32_t i = (literal ? chunk : chunk - literal_chunks) * 32U + static_cast<uint32_t>(lane);
     bool updated = false;
     uint32_t newly = 0U;
-    if (i < n) {
-      const uint32_t code = V.active[i];
+    if (i < (literal ? n_literal : n)) {
+      const uint32_t code = V.active[literal ? last - i : i];
       const uint32_t b = code >> 9;
       const int li = static_cast<int>(code & 511U);
       const int4 bk = V.block_keys[b];
       f3 pc;
-      float u, v, d;
-      voxel_prefix(depth, p, bk, li, pc, u, v, d);
+      float u, v;
+      voxel_projection(p, bk, li, pc, u, v);
       float sc = 0.0f, obs = 0.0f;
       f3 spw = mk3(0.0f, 0.0f, 0.0f), nw = spw;
-      const int dir = voxel_observation<kUpdateThreads>(depth, p, pc, u, v, d, gs, S, threadIdx.x, sc, spw, nw, obs);
+      const int dir = voxel_observation<kUpdateThreads>(depth, p, cam, pc, u, v, literal, gs, S, threadIdx.x, sc, spw,
+                                                        nw, obs);
       if (dir >= 0) {
         float4 L0, L1, L2;
-        load_bin(V, b, dir, li, bk, p.voxel_size, L0, L1, L2);
+        if (kFp16) {
+          load_bin(V, b, dir, li, bk, p.voxel_size, L0, L1, L2);
+        } else {
+          const float4* bin = V.layers + layer_index(b, dir, li, 0);
+          L0 = bin[0];
+          L1 = bin[1];
+          L2 = bin[2];
+        }
         updated = integrate_sample(p, L0, L1, L2, sc, spw, nw, obs);
         if (updated) {
-          store_bin(V, b, dir, li, bk, p.voxel_size, L0, L1, L2);
+          if (kFp16) {
+            store_bin(V, b, dir, li, bk, p.voxel_size, L0, L1, L2);
+          } else {
+            float4* bin = V.layers + layer_index(b, dir, li, 0);
+            bin[0] = L0;
+            bin[1] = L1;
+            bin[2] = L2;
+          }
           const size_t w = static_cast<size_t>(b) * (kBlockVoxels / 32) + (li >> 5);
           const uint32_t bit = 1U << (li & 31);
           if (!(V.obs_mask[w] & bit)) newly = (atomicOr(&V.obs_mask[w], bit) & bit) ? 0U : 1U;
@@ -637,12 +799,12 @@ __global__ void __launch_bounds__(kUpdateThreads) update_kernel(const float* __r
         }
       }
     }
-    const uint32_t upd = __ballot_sync(0xffffffffU, updated);
-    const uint32_t nw_ = __ballot_sync(0xffffffffU, newly != 0U);
-    if (lane == 0) {
-      if (upd) atomicAdd(&V.counters->integrated_voxels, static_cast<uint32_t>(__popc(upd)));
-      if (nw_) atomicAdd(&V.counters->observed_voxels, static_cast<unsigned long long>(__popc(nw_)));
-    }
+    sum_updated += static_cast<uint32_t>(__popc(__ballot_sync(0xffffffffU, updated)));
+    sum_newly += static_cast<uint32_t>(__popc(__ballot_sync(0xffffffffU, newly != 0U)));
+  }
+  if (lane == 0) {  // once per warp: the counters share one L2 line
+    if (sum_updated) atomicAdd(&V.counters->integrated_voxels, sum_updated);
+    if (sum_newly) atomicAdd(&V.counters->observed_voxels, static_cast<unsigned long long>(sum_newly));
   }
 }
 
@@ -1389,7 +1551,7 @@ static int grid_for(const void* kernel, int threads) {
 
 int integrate_grid_size() {
   static int grid = 0;
-  if (grid == 0) grid = grid_for(reinterpret_cast<const void*>(update_kernel), kUpdateThreads);
+  if (grid == 0) grid = grid_for(reinterpret_cast<const void*>(update_kernel<false>), kUpdateThreads);
   return grid;
 }
 
@@ -1484,7 +1646,12 @@ cudaError_t launch_integrate_update(const float* depth, const Volume& V, const P
     fv.launch(grid > 0 ? grid : fused_grid[variant], s, depth, nmap, V, p);
     return cudaGetLastError();
   }
-  update_kernel<<<grid > 0 ? grid : integrate_grid_size(), kUpdateThreads, 0, s>>>(depth, V, p);
+  const int g = grid > 0 ? grid : integrate_grid_size();
+  if (V.layers16 != nullptr) {
+    update_kernel<true><<<g, kUpdateThreads, 0, s>>>(depth, V, p);
+  } else {
+    update_kernel<false><<<g, kUpdateThreads, 0, s>>>(depth, V, p);
+  }
   return cudaGetLastError();
 }
 
