@@ -54,3 +54,34 @@ def test_raycast_remainder_tiles_bit_exact(env, small_orbit, fp16, size, step):
         assert np.array_equal(_bits(got), _bits(ora.raycast_depth(K, pose, 0.0, 3.0, step)))
     vol.close()
     ora.close()
+
+
+@pytest.mark.parametrize("offset", [0, 4])
+@pytest.mark.parametrize("fp16", [0, 1])
+def test_export_to_device_equals_host(env, small_orbit, fp16, offset):
+    """Blocks exported into device memory, directly (16-byte aligned) and through the staging buffer (4 bytes off), equal
+    the host export word for word: the whole pool (over one staging pass), a range inside it, keys or voxels alone."""
+    backend, O = env
+    from voxelhashmt_gb300 import _capi
+    vol, ora = _fuse(backend, O, small_orbit, [0, 5, 10, 15], fp16)
+    n = vol.block_count()
+    assert n > 1024 or fp16
+    for first, count in ((0, n), (3, 1), (n - 77, 77)):
+        hk, hv = vol.export_blocks(first, count)
+        words = count * 512 * 6 * 3 * 4
+        buf = torch.zeros(words + 4, dtype=torch.int32, device="cuda")
+        keys = torch.zeros((count, 3), dtype=torch.int32, device="cuda")
+        kp, vp = C.cast(C.c_void_p(keys.data_ptr()), C.POINTER(C.c_int32)), C.c_void_p(buf.data_ptr() + offset)
+        for k, v in ((kp, vp), (kp, None), (None, vp)):
+            buf.zero_()
+            keys.zero_()
+            _capi.check(_capi.lib().vh_export_blocks(vol.handle, first, count, k, v, 1, None), vol.handle)
+            got = buf[offset // 4:offset // 4 + words].cpu().numpy().view(np.uint32)
+            assert np.array_equal(got, hv.reshape(-1) if v else np.zeros_like(got))
+            assert np.array_equal(keys.cpu().numpy(), hk if k else np.zeros_like(hk))
+    gk, gv = O.sort_blocks(*vol.export_blocks())
+    ok, ov = O.sort_blocks(*ora.blocks())
+    assert np.array_equal(gk, ok)
+    assert np.array_equal(gv.reshape(len(gk), -1), ov.view(np.uint32).reshape(len(ok), -1))
+    vol.close()
+    ora.close()

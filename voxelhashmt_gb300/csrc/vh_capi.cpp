@@ -2,6 +2,7 @@
 //
 // Host code is compiled with -ffp-contract=off: the world->camera pose (Pose::inverse, math_types.h:192-197)
 // and the 1/(2 sigma^2) factors are float expressions whose rounding must match the reference's.
+#include <cuda.h>  // the address-range query's types (resolved at run time, no link dependency)
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -271,6 +272,37 @@ vh_status stage_release(vh_volume* v, int slot, cudaStream_t s) {
   VH_CUDA(v, cudaEventRecord(v->stage_free[slot], s));
   v->stage_used[slot] = true;
   return VH_OK;
+}
+
+// memory of the volume's device (or managed memory) aligned to `align` bytes, or no pointer: a kernel may store into
+// it; anything else goes through cudaMemcpy
+bool device_memory(const vh_volume* v, const void* ptr, size_t align) {
+  if (!ptr) return true;
+  if (reinterpret_cast<uintptr_t>(ptr) % align != 0) return false;
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, ptr) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return (at.type == cudaMemoryTypeDevice && at.device == v->params.device) || at.type == cudaMemoryTypeManaged;
+}
+
+// `bytes` from ptr lie inside one allocation of the current device: a kernel's stores past its end would be a fault
+// where cudaMemcpy returns an error
+bool inside_allocation(const void* ptr, size_t bytes) {
+  if (!ptr) return true;
+  using RangeFn = CUresult (*)(CUdeviceptr*, size_t*, CUdeviceptr);
+  static const RangeFn range = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult qr = cudaDriverEntryPointSymbolNotFound;
+    const cudaError_t e = cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &fn, 12000, cudaEnableDefault, &qr);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e == cudaSuccess && qr == cudaDriverEntryPointSuccess ? reinterpret_cast<RangeFn>(fn) : nullptr;
+  }();
+  CUdeviceptr base = 0;
+  size_t size = 0;
+  const auto p = static_cast<CUdeviceptr>(reinterpret_cast<uintptr_t>(ptr));
+  return range && range(&base, &size, p) == CUDA_SUCCESS && p - base <= size && bytes <= size - (p - base);
 }
 
 uint64_t block_total(const vh_volume* v) {
@@ -806,18 +838,7 @@ vh_status vh_evict_blocks(vh_volume* v, uint32_t min_age_frames, uint64_t target
   // 1. copy the victims out: into device memory directly (16-byte aligned), else through the staging buffer
   const size_t bytes = format == 1 ? native_block_bytes(v) : kBlockBytes;
   const cudaMemcpyKind kind = out_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
-  // device (or managed) memory only: the copy kernel then stores into it; anything else goes through cudaMemcpy
-  auto device_memory = [](const void* ptr) {
-    if (!ptr) return true;
-    cudaPointerAttributes at{};
-    if (cudaPointerGetAttributes(&at, ptr) != cudaSuccess) {
-      cudaGetLastError();
-      return false;
-    }
-    return at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged;
-  };
-  const bool direct = out_on_device && reinterpret_cast<uintptr_t>(data_out) % 16 == 0 && device_memory(data_out) &&
-                      device_memory(keys_out);
+  const bool direct = out_on_device && device_memory(v, data_out, 16) && device_memory(v, keys_out, 4);
   if (keys_out || data_out) {
     for (uint64_t done = 0; done < nv; done += kExportChunk) {
       const uint32_t c = static_cast<uint32_t>(std::min<uint64_t>(kExportChunk, nv - done));
@@ -1219,6 +1240,15 @@ vh_status vh_export_blocks(vh_volume* v, uint64_t first, uint64_t count, int32_t
   if (st != VH_OK) return st;
   if (first + count > block_total(v)) return fail(v, VH_ERR_INVALID_ARGUMENT, "vh_export_blocks: range beyond block count");
   if (count == 0 || (!keys && !voxels)) return VH_OK;
+  if (on_device && device_memory(v, voxels, 16) && device_memory(v, keys, 4) &&
+      inside_allocation(voxels, count * kBlockBytes) && inside_allocation(keys, 3 * count * sizeof(int32_t))) {
+    // the kernel stores into the caller's buffers: through the staging buffer the records were written twice and
+    // read once more
+    VH_CUDA(v, vh::launch_export(v->dev, nullptr, static_cast<uint32_t>(first), static_cast<uint32_t>(count), keys,
+                                 static_cast<float4*>(voxels), s));
+    VH_CUDA(v, cudaStreamSynchronize(s));
+    return VH_OK;
+  }
   if (!v->d_export) {
     VH_CUDA(v, cudaMalloc(reinterpret_cast<void**>(&v->d_export), kExportChunk * kBlockBytes));
     VH_CUDA(v, dalloc(&v->d_export_keys, 3 * kExportChunk));
@@ -1227,7 +1257,8 @@ vh_status vh_export_blocks(vh_volume* v, uint64_t first, uint64_t count, int32_t
   const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
   for (uint64_t done = 0; done < count; done += kExportChunk) {
     const uint32_t n = static_cast<uint32_t>(std::min<uint64_t>(kExportChunk, count - done));
-    VH_CUDA(v, vh::launch_export(v->dev, static_cast<uint32_t>(first + done), n, v->d_export_keys, v->d_export, s));
+    VH_CUDA(v, vh::launch_export(v->dev, nullptr, static_cast<uint32_t>(first + done), n,
+                                 keys ? v->d_export_keys : nullptr, voxels ? v->d_export : nullptr, s));
     if (voxels) {
       VH_CUDA(v, cudaMemcpyAsync(static_cast<char*>(voxels) + done * kBlockBytes, v->d_export, n * kBlockBytes, kind, s));
     }

@@ -157,32 +157,6 @@ __global__ void __launch_bounds__(256) copy_out_native_kernel(const Volume V, co
   }
 }
 
-// listed blocks in the reference Voxel layout voxels[i][li][d][l] (decoded FP16 bins) and keys
-__global__ void __launch_bounds__(256) copy_out_reference_kernel(const Volume V, const uint32_t* __restrict__ list,
-                                                                 uint32_t n, int* __restrict__ keys,
-                                                                 float4* __restrict__ out) {
-  const size_t total = static_cast<size_t>(n) * kBlockVoxels * kDirs;
-  for (size_t t = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; t < total;
-       t += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    const int d = static_cast<int>(t % kDirs);
-    const int li = static_cast<int>((t / kDirs) % kBlockVoxels);
-    const uint32_t i = static_cast<uint32_t>(t / (static_cast<size_t>(kDirs) * kBlockVoxels));
-    const uint32_t b = list[i];
-    const int4 bk = V.block_keys[b];
-    float4 L0, L1, L2;
-    load_bin(V, b, d, li, bk, V.voxel_size, L0, L1, L2);
-    float4* o = out + t * kLayers;
-    o[0] = L0;
-    o[1] = L1;
-    o[2] = L2;
-    if (d == 0 && li == 0) {
-      keys[3 * i] = bk.x;
-      keys[3 * i + 1] = bk.y;
-      keys[3 * i + 2] = bk.z;
-    }
-  }
-}
-
 // block src[i] -> dst[i] with its key, masks and stamp: one CTA per move
 // observed voxels of the victims (set bits of their observed-voxel masks; a bit is set exactly when the voxel
 // has a layer of positive weight), subtracted from the volume's count once the victims are gone: the same
@@ -301,7 +275,7 @@ cudaError_t launch_copy_out(const Volume& V, const uint32_t* list, uint32_t n, i
   if (native) {
     copy_out_native_kernel<<<152 * 4, 256, 0, s>>>(V, list, n, keys, static_cast<uint4*>(out));
   } else {
-    copy_out_reference_kernel<<<152 * 8, 256, 0, s>>>(V, list, n, keys, static_cast<float4*>(out));
+    return launch_export(V, list, 0U, n, keys, static_cast<float4*>(out), s);
   }
   return cudaGetLastError();
 }

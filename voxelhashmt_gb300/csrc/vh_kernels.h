@@ -80,10 +80,11 @@ int mc_grid_size();
 cudaError_t launch_recount(const Volume& V, unsigned long long* out, cudaStream_t s);
 // keys of the current frame's visible blocks (int3 each, unordered)
 cudaError_t launch_visible_keys(const Volume& V, int* keys, cudaStream_t s);
-// copy blocks [first, first+count) to the reference layout: keys int32[count][3],
-// voxels [count][512][6][3] x {f32 weight, f32 surface_coord, f32 plane_offset, u32 packed_normal}
-cudaError_t launch_export(const Volume& V, uint32_t first, uint32_t count, int* keys, float4* voxels,
-                          cudaStream_t s);
+// copy blocks [first, first+count), or the listed ones (list: count pool indices), to the reference layout: keys
+// int32[count][3], voxels [count][512][6][3] x {f32 weight, f32 surface_coord, f32 plane_offset, u32 packed_normal};
+// either may be null
+cudaError_t launch_export(const Volume& V, const uint32_t* list, uint32_t first, uint32_t count, int* keys,
+                          float4* voxels, cudaStream_t s);
 
 // import blocks in the reference layout (insert or overwrite); idx: n scratch words
 cudaError_t launch_import(const Volume& V, const int* keys, const float4* voxels, uint32_t n, uint32_t* idx,
