@@ -85,3 +85,51 @@ def test_export_to_device_equals_host(env, small_orbit, fp16, offset):
     assert np.array_equal(gv.reshape(len(gk), -1), ov.view(np.uint32).reshape(len(ok), -1))
     vol.close()
     ora.close()
+
+
+def _random_blocks(rng, keys, vs, fill):
+    """Records (N, 512, 6, 3, 4) of random layers: a share `fill` of them observed, planes within 2 voxels of their
+    voxel, normals in any direction."""
+    n = len(keys)
+    li = np.arange(512)
+    local = np.stack([li & 7, (li >> 3) & 7, li >> 6], -1)
+    centre = ((np.asarray(keys)[:, None, :] * 8 + local[None]) + 0.5) * vs  # (N, 512, 3)
+    nrm = rng.normal(size=(n, 512, 6, 3, 3))
+    nrm /= np.linalg.norm(nrm, axis=-1, keepdims=True)
+    oct_ = nrm[..., :2] / np.abs(nrm).sum(-1, keepdims=True)
+    sign = np.where(oct_ >= 0, 1.0, -1.0)
+    oct_ = np.where(nrm[..., 2:] < 0, (1 - np.abs(oct_[..., ::-1])) * sign, oct_)
+    q = np.floor((oct_ * 0.5 + 0.5) * 65535 + 0.5).astype(np.uint32)
+    vox = np.zeros((n, 512, 6, 3, 4), np.float32)
+    seen = rng.random((n, 512, 6, 3)) < fill
+    offset = np.einsum("nvdlk,nvk->nvdl", nrm, centre) + rng.uniform(-2, 2, (n, 512, 6, 3)) * vs
+    vox[..., 0] = np.where(seen, rng.uniform(0.1, 50.0, seen.shape), 0.0)
+    vox[..., 1] = np.where(seen, centre[..., None, None, 0] + rng.uniform(-1, 1, seen.shape) * vs, 0.0)
+    vox[..., 2] = np.where(seen, offset, 0.0)
+    out = vox.view(np.uint32)
+    out[..., 3] = np.where(seen, q[..., 0] | (q[..., 1] << 16), 0)
+    return out
+
+
+@pytest.mark.parametrize("fp16", [0, 1])
+@pytest.mark.parametrize("fill,iso", [(0.02, 0.0), (0.35, 0.0), (0.9, 0.004)])
+def test_mesh_of_random_layers(env, fp16, fill, iso):
+    """Marching cubes of blocks of random planes against the oracle: from nearly empty blocks to every cell marked in
+    every direction with up to 24 candidates, blocks alone and touching on faces, edges and corners, negative and large
+    coordinates, an iso level off 0."""
+    backend, O = env
+    vs = 0.02
+    keys = np.array([[x, y, z] for x in (-1, 0) for y in (-1, 0) for z in (-1, 0)] +
+                    [[5, 5, 5], [6, 6, 6], [7, 6, 5], [-40, 3, 0], [300, -200, 100]], np.int32)
+    vox = _random_blocks(np.random.default_rng(int(100 * fill)), keys, vs, fill)
+    vol = backend.VoxelHashTSDF(vs, 4 * vs, hash_buckets=1 << 10, max_blocks=len(keys), layer_format=fp16)
+    ora = O.Volume(O.config(O.FLAVOR_REF_GPU, O.EXP_OWN, threads=8, layer_format=fp16), vs, 4 * vs)
+    vol.import_blocks(keys, vox)
+    ora.apply_flat_blocks(keys, vox)
+    tris = backend.extract_mesh_cuda(vol, iso)
+    want = ora.extract_mesh(iso)
+    assert tris.shape == want.shape and (fill < 0.1 or tris.shape[0] > 100)
+    assert np.array_equal(_bits(O.canonical_triangles(tris)), _bits(O.canonical_triangles(want)))
+    assert np.array_equal(_bits(backend.extract_mesh_cuda(vol, iso)), _bits(tris))  # the same order every time
+    vol.close()
+    ora.close()

@@ -50,10 +50,8 @@ struct vh_volume {
   std::vector<int> tune_variant_of;
   float tune_best_ms = 0.0f;
   size_t depth_capacity = 0;  // pixels
-  uint32_t* d_mc_counts = nullptr;
-  uint32_t* d_mc_dir_totals = nullptr;
-  uint8_t* d_mc_cell_counts = nullptr;
-  unsigned long long* d_mc_offsets = nullptr;
+  vh::MeshBuffers mc{};
+  uint32_t mc_epoch = 0;  // of the last incremental extraction
   uint32_t* d_mc_list = nullptr;        // incremental meshing: the selected pool blocks
   uint32_t* d_mc_list_count = nullptr;
   unsigned long long* d_scalar = nullptr;  // [0] mesh total, [1] recount
@@ -385,6 +383,36 @@ void free_weld(vh_volume* v) {
   v->weld_capacity = 0;
 }
 
+void free_mesh(vh_volume* v) {
+  vh::MeshBuffers& M = v->mc;
+  M.neighbours = M.cell_mask = M.rounds = nullptr;  // parts of the active list
+  dfree(M.cell_counts);
+  dfree(M.dir_totals);
+  dfree(M.offsets);
+  dfree(M.need);
+  dfree(M.queue);
+}
+
+vh_status ensure_mesh(vh_volume* v) {
+  vh::MeshBuffers& M = v->mc;
+  if (M.queue) return VH_OK;
+  const size_t n = v->dev.max_blocks;
+  free_mesh(v);  // what an attempt that ran out of memory left
+  // The active list (512 words per block) is scratch of one frame's update, on the volume's one stream at a time: the
+  // rounds, cell masks and neighbours of an extraction (96 + 96 + 8 words per block) use it in between.
+  const size_t words = vh::kDirs * (vh::kBlockVoxels / 32);
+  M.rounds = v->dev.active;
+  M.cell_mask = v->dev.active + n * words;
+  M.neighbours = v->dev.active + 2 * n * words;
+  VH_CUDA(v, dalloc(&M.cell_counts, n * vh::kDirs * vh::kBlockVoxels));
+  VH_CUDA(v, dalloc(&M.dir_totals, n * vh::kDirs));
+  VH_CUDA(v, dalloc(&M.offsets, n));
+  VH_CUDA(v, dalloc(&M.need, n));
+  VH_CUDA(v, cudaMemset(M.need, 0, n * sizeof(uint32_t)));
+  VH_CUDA(v, dalloc(&M.queue, 4));
+  return VH_OK;
+}
+
 // weld buffers for a soup of `triangles` triangles (3 * triangles < 2^30)
 vh_status ensure_weld(vh_volume* v, size_t triangles) {
   if (triangles <= v->weld_capacity && v->weld.counts) return VH_OK;
@@ -615,10 +643,7 @@ void vh_destroy(vh_volume* v) {
     cudaEventDestroy(pair[0]);
     cudaEventDestroy(pair[1]);
   }
-  dfree(v->d_mc_counts);
-  dfree(v->d_mc_dir_totals);
-  dfree(v->d_mc_cell_counts);
-  dfree(v->d_mc_offsets);
+  free_mesh(v);
   dfree(v->d_mc_list);
   dfree(v->d_mc_list_count);
   dfree(v->d_scalar);
@@ -1057,12 +1082,8 @@ static vh_status extract(vh_volume* v, float iso, uint32_t frames, size_t* trian
   if (!v || !triangle_count || v->dev.max_blocks == 0) return fail(v, VH_ERR_INVALID_ARGUMENT, "vh_extract_mesh: bad argument");
   DeviceGuard guard(v->params.device);
   const cudaStream_t s = as_stream(stream);
-  if (!v->d_mc_counts) {
-    VH_CUDA(v, dalloc(&v->d_mc_counts, v->dev.max_blocks));
-    VH_CUDA(v, dalloc(&v->d_mc_offsets, v->dev.max_blocks));
-    VH_CUDA(v, dalloc(&v->d_mc_dir_totals, static_cast<size_t>(v->dev.max_blocks) * vh::kDirs));
-    VH_CUDA(v, dalloc(&v->d_mc_cell_counts, static_cast<size_t>(v->dev.max_blocks) * vh::kDirs * vh::kBlockVoxels));
-  }
+  const vh_status st = ensure_mesh(v);
+  if (st != VH_OK) return st;
   const uint32_t* list = nullptr;
   const uint32_t* list_count = nullptr;
   if (frames > 0) {
@@ -1071,17 +1092,17 @@ static vh_status extract(vh_volume* v, float iso, uint32_t frames, size_t* trian
       VH_CUDA(v, dalloc(&v->d_mc_list_count, 1));
     }
     VH_CUDA(v, vh::launch_recent_blocks(v->dev, frames, v->d_mc_list, v->d_mc_list_count, s));
-    // blocks outside the list contribute nothing to the scan
-    VH_CUDA(v, cudaMemsetAsync(v->d_mc_counts, 0, static_cast<size_t>(v->dev.max_blocks) * sizeof(uint32_t), s));
+    if (++v->mc_epoch == 0U) {  // wrapped: no stamp of an earlier call may be taken for this one's
+      VH_CUDA(v, cudaMemsetAsync(v->mc.need, 0, static_cast<size_t>(v->dev.max_blocks) * sizeof(uint32_t), s));
+      v->mc_epoch = 1U;
+    }
     list = v->d_mc_list;
     list_count = v->d_mc_list_count;
   }
   vh_intrinsics K{1, 1, 1.0f, 1.0f, 0.0f, 0.0f};
   vh::Params p = make_params(v, &K, nullptr, 1);
   p.iso = iso;
-  VH_CUDA(v, vh::launch_mc_count(v->dev, p, v->d_mc_counts, v->d_mc_dir_totals, v->d_mc_cell_counts, list, list_count,
-                                 s));
-  VH_CUDA(v, vh::launch_mc_scan(v->dev, v->d_mc_counts, v->d_mc_offsets, v->d_scalar, s));
+  VH_CUDA(v, vh::launch_mc_count(v->dev, p, v->mc, list, list_count, v->mc_epoch, v->d_scalar, s));
   unsigned long long total = 0;
   VH_CUDA(v, cudaMemcpyAsync(&total, v->d_scalar, sizeof(total), cudaMemcpyDeviceToHost, s));
   VH_CUDA(v, cudaStreamSynchronize(s));
@@ -1093,8 +1114,7 @@ static vh_status extract(vh_volume* v, float iso, uint32_t frames, size_t* trian
     v->tri_capacity = cap;
   }
   if (total > 0) {
-    VH_CUDA(v, vh::launch_mc_emit(v->dev, p, v->d_mc_counts, v->d_mc_dir_totals, v->d_mc_cell_counts,
-                                  v->d_mc_offsets, v->d_tris, list, list_count, s));
+    VH_CUDA(v, vh::launch_mc_emit(v->dev, p, v->mc, v->d_tris, s));
   }
   VH_CUDA(v, cudaStreamSynchronize(s));
   v->mesh_triangles = static_cast<size_t>(total);

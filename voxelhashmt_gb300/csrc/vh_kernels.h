@@ -63,19 +63,27 @@ void fused_variant_shape(int variant, int* threads, int* min_blocks);
 cudaError_t launch_pixel_normals(const float* depth, const Params& p, float4* nmap, cudaStream_t s);
 int integrate_grid_size();
 }  // namespace fast
-// marching cubes over all allocated blocks (or the blocks of `list`, *list_count entries, device memory): pass 1
-// writes per-block, per-direction and per-cell triangle
-// counts, the scan turns the block counts into offsets (+ total), pass 2 writes triangles (9 floats each)
-cudaError_t launch_mc_count(const Volume& V, const Params& p, uint32_t* counts, uint32_t* dir_totals,
-                            uint8_t* cell_counts, const uint32_t* list, const uint32_t* list_count, cudaStream_t s);
+// marching cubes over all allocated blocks (or the blocks of `list`, *list_count entries, device memory).  Buffers for
+// max_blocks blocks: neighbours 8 words per block, cell_mask 6 x 16 words, cell_counts 6 x 512 bytes, dir_totals 6
+// words, offsets 1 u64, need 1 word (zeroed once; each list call with another epoch > 0), rounds 6 x 16 words; queue
+// 4 words.
+// launch_mc_count leaves the cells with triangles, their counts and offsets, and the triangle total; launch_mc_emit
+// writes the triangles (9 floats each).
+struct MeshBuffers {
+  uint32_t* neighbours;
+  uint32_t* cell_mask;
+  uint8_t* cell_counts;
+  uint32_t* dir_totals;
+  unsigned long long* offsets;
+  uint32_t* need;
+  uint32_t* rounds;
+  uint32_t* queue;
+};
+cudaError_t launch_mc_count(const Volume& V, const Params& p, const MeshBuffers& M, const uint32_t* list,
+                            const uint32_t* list_count, uint32_t epoch, unsigned long long* total, cudaStream_t s);
 // pool blocks updated within the last `frames` frames -> list (count on the device, reset here)
 cudaError_t launch_recent_blocks(const Volume& V, uint32_t frames, uint32_t* list, uint32_t* count, cudaStream_t s);
-cudaError_t launch_mc_scan(const Volume& V, const uint32_t* counts, unsigned long long* offsets,
-                           unsigned long long* total, cudaStream_t s);
-cudaError_t launch_mc_emit(const Volume& V, const Params& p, const uint32_t* counts, const uint32_t* dir_totals,
-                           const uint8_t* cell_counts, const unsigned long long* offsets, float* tris,
-                           const uint32_t* list, const uint32_t* list_count, cudaStream_t s);
-int mc_grid_size();
+cudaError_t launch_mc_emit(const Volume& V, const Params& p, const MeshBuffers& M, float* tris, cudaStream_t s);
 // full recount of observed voxels (any layer weight > 0) over the pool
 cudaError_t launch_recount(const Volume& V, unsigned long long* out, cudaStream_t s);
 // keys of the current frame's visible blocks (int3 each, unordered)
