@@ -133,3 +133,48 @@ def test_mesh_of_random_layers(env, fp16, fill, iso):
     assert np.array_equal(_bits(backend.extract_mesh_cuda(vol, iso)), _bits(tris))  # the same order every time
     vol.close()
     ora.close()
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (2, 5, 33), (1, 17, 30), (1, 14, 61), (3, 16, 32), (1, 40, 100)])
+def test_denoiser_layers_at_tile_edges(env, shape):
+    """The denoiser's output and every gradient on images smaller than a tile, with remainders of the 32x16, 30x14 and
+    32x8 tiles and pixels without depth, against float64 with BF16 rounding where the kernels store BF16.  Output:
+    FP32 sums may round an activation to the other BF16 neighbour, 2^-8 of it, in each of the three layers; the bound
+    carries that through the magnitudes of the weights (plus 1e-6 m of FP32 rounding).  Gradients: each parameter group
+    within 2 % relative L2, as for the larger images of test_gpu_nn.py."""
+    import torch.nn.functional as F
+    from tests.test_gpu_nn import _ref_loss
+    from voxelhashmt_gb300 import denoiser
+    b, h, w = shape
+    rng = np.random.default_rng(b * 100 + h * 10 + w)
+    yy, xx = np.meshgrid(np.arange(h), np.arange(w), indexing="ij")
+    clean = (1.5 + 0.01 * yy + 0.005 * xx)[None] + rng.uniform(0, 0.5, (b, 1, 1))
+    raw = (clean + rng.normal(0, 0.003, (b, h, w))).astype(np.float32)
+    if h * w > 1:
+        raw[rng.random((b, h, w)) < 0.1] = 0.0
+    p0 = denoiser.init_params(seed=5)
+    p0[-289:] = rng.normal(0, 0.05, 289).astype(np.float32)
+    net = denoiser.DepthDenoiser(p0)
+    got, _, out = net.gradients(torch.from_numpy(raw).cuda(), torch.from_numpy(clean.astype(np.float32)).cuda())
+    params = torch.from_numpy(p0.astype(np.float64)).requires_grad_(True)
+    loss, want = _ref_loss(params, torch.from_numpy(raw).double(), torch.from_numpy(clean.astype(np.float32)).double())
+    loss.backward()
+    ref = params.grad.numpy()
+    want = want.detach().numpy()
+    # magnitudes of the activations and of what one rounding step per activation can move, layer by layer
+    w1, b1, w2, b2, w3, b3, w4, _ = torch.split(params.detach().abs(), [1152, 32, 9216, 32, 9216, 32, 288, 1])
+    d = torch.from_numpy(raw).double().unsqueeze(1)
+    x = torch.cat([torch.full_like(d, 100 * 0.06), torch.ones_like(d), torch.ones_like(d), 0 * d], 1)  # bounds the channels
+    mag, err = x, 0 * x
+    for wt, bt, cin in ((w1, b1, 4), (w2, b2, 32), (w3, b3, 32)):
+        wt = wt.view(32, cin, 3, 3)
+        err = F.conv2d(err, wt, padding=1)
+        mag = F.conv2d(mag, wt, bt, padding=1)
+        err = err + 2.0 ** -8 * mag
+    tol = (0.01 * F.conv2d(err, w4.view(1, 32, 3, 3), padding=1)).squeeze(1).numpy() + 1e-6
+    assert np.all(np.abs(out.cpu().numpy().reshape(want.shape) - want) <= tol)
+    off = 0
+    for n in (32 * 4 * 9, 32, 32 * 32 * 9, 32, 32 * 32 * 9, 32, 32 * 9, 1):
+        a, r = got[off:off + n].astype(np.float64), ref[off:off + n]
+        assert np.linalg.norm(a - r) <= 2e-2 * np.linalg.norm(r) + 1e-12, (off, n)
+        off += n

@@ -18,7 +18,8 @@
 // The input gradient of a 32 -> 32 layer is the same convolution with the weights flipped in space and
 // transposed in channels, so the backward pass reuses the kernel.  The weight gradient of a 32 -> 32 layer (a
 // reduction over pixels) is a second tensor-core kernel, wgrad32_tc_kernel.  The 4-channel input layer, the
-// 1-channel output layer, their weight gradients and Adam run on the CUDA cores in FP32.
+// 1-channel output layer, their weight gradients and Adam run on the CUDA cores in FP32, the input channels always
+// computed from the depth where they are used.
 //
 // Safety: the descriptors address only staged bytes: an A operand reads at most 8,608 bytes into its 8,704-byte
 // slot (pixels dx .. dx + 127 of each plane), the B operand exactly kBBytes, followed by a margin; the layout is
@@ -555,8 +556,8 @@ cudaError_t launch_pack_w32(const float* w, __nv_bfloat16* out, int transpose_fl
 // slot the gradient ring that follows: staged values, finite, feeding only accumulator rows that are never
 // read.  The gradient row is staged the same way as the B operand, [pixel group][output channel][8 pixels].  A
 // thread loads a channel pair over 10 (8) pixels as 32-bit words and writes the transposed 16-byte rows with
-// byte permutes; the loads of a row are issued before the wait for its ring slot, so they overlap the MMAs
-// that still read the slot.  Rows live in rings (three input rows, two gradient rows); thread 0 issues an output
+// byte permutes; the loads of a row are issued a row ahead, so they are in flight while the row before it is
+// staged and multiplied (a batch of 16 640x480 frames: 374 -> 287 us, shared-memory traffic now the largest part).  Rows live in rings (three input rows, two gradient rows); thread 0 issues an output
 // row's 12 MMAs (3 tap rows x 4 k-steps of 16 pixels) and commits them to an mbarrier, and a ring slot is
 // rewritten only after the MMAs that read it have completed.  Four CTAs per SM (their tensor memory fills the
 // SM's 512 columns).  Waits are bounded as in conv32_tc_kernel; a timeout is agreed on by every thread
@@ -642,38 +643,52 @@ __global__ void __launch_bounds__(kWgThreads, kWgCtasPerSm) wgrad32_tc_kernel(co
     }
   };
 
-  for (uint32_t it = blockIdx.x; it < nitems && ok; it += gridDim.x) {
+  // the words of input row y0 + i + 1 and, for i >= 0, gradient row y0 + i of an item
+  auto load_rows = [&](uint32_t it, int i, uint32_t (&wv)[10], uint32_t (&gv)[8]) {
     const uint32_t rest = it / strips;
     const int xs = static_cast<int>(it - rest * strips) * kWgStrip;
     const uint32_t img = rest / rblocks;
     const int y0 = static_cast<int>(rest - img * rblocks) * kWgRows;
+    const size_t img_base = static_cast<size_t>(img) * height;
+    const int y = y0 + i + 1;
+    const bool rok = y >= 0 && y < height;
+    const unsigned int* rowp = reinterpret_cast<const unsigned int*>(X + (img_base + (rok ? y : 0)) * width * kC) + cp;
+#pragma unroll
+    for (int j = 0; j < 10; ++j) {
+      const int px = xs - 1 + 8 * pg + j;
+      wv[j] = (rok && px >= 0 && px < width) ? __ldg(rowp + static_cast<size_t>(px) * (kC / 2)) : 0u;
+    }
+    if (i >= 0) {
+      const unsigned int* growp = reinterpret_cast<const unsigned int*>(G + (img_base + (y0 + i)) * width * kC) + cp;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int px = xs + 8 * pg + j;
+        gv[j] = px < width ? __ldg(growp + static_cast<size_t>(px) * (kC / 2)) : 0u;
+      }
+    }
+  };
+  uint32_t nwv[10], ngv[8];  // the next row's words: in flight while this row is staged and multiplied
+#pragma unroll
+  for (int j = 0; j < 8; ++j) ngv[j] = 0u;
+  if (blockIdx.x < nitems) load_rows(blockIdx.x, -2, nwv, ngv);
+
+  for (uint32_t it = blockIdx.x; it < nitems && ok; it += gridDim.x) {
+    const uint32_t rest = it / strips;
+    const uint32_t img = rest / rblocks;
+    const int y0 = static_cast<int>(rest - img * rblocks) * kWgRows;
     const int rows = min(kWgRows, height - y0);
     const uint32_t xa = xq;  // ring index of input row y0 - 1
-    const size_t img_base = static_cast<size_t>(img) * height;
     for (int i = -2; i < rows; ++i) {
-      // stage input row y0 + i + 1 and, for i >= 0, gradient row y0 + i; then issue output row y0 + i.  The
-      // global loads go first: they do not touch the rings, so they overlap the wait for the slots.
-      const int y = y0 + i + 1;
-      uint32_t wv[10];
-      {
-        const bool rok = y >= 0 && y < height;
-        const unsigned int* rowp =
-            reinterpret_cast<const unsigned int*>(X + (img_base + (rok ? y : 0)) * width * kC) + cp;
+      // stage input row y0 + i + 1 and, for i >= 0, gradient row y0 + i; then issue output row y0 + i
+      uint32_t wv[10], gv[8];
 #pragma unroll
-        for (int j = 0; j < 10; ++j) {
-          const int px = xs - 1 + 8 * pg + j;
-          wv[j] = (rok && px >= 0 && px < width) ? __ldg(rowp + static_cast<size_t>(px) * (kC / 2)) : 0u;
-        }
-      }
-      uint32_t gv[8];
-      if (i >= 0) {
-        const unsigned int* growp =
-            reinterpret_cast<const unsigned int*>(G + (img_base + (y0 + i)) * width * kC) + cp;
+      for (int j = 0; j < 10; ++j) wv[j] = nwv[j];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int px = xs + 8 * pg + j;
-          gv[j] = px < width ? __ldg(growp + static_cast<size_t>(px) * (kC / 2)) : 0u;
-        }
+      for (int j = 0; j < 8; ++j) gv[j] = ngv[j];
+      if (i + 1 < rows) {
+        load_rows(it, i + 1, nwv, ngv);
+      } else if (it + gridDim.x < nitems) {
+        load_rows(it + gridDim.x, -2, nwv, ngv);
       }
       const uint32_t sx = xq % kWgXSlots;
       if (reader[sx] >= 0) wait_through(reader[sx]);
@@ -819,348 +834,587 @@ __device__ __forceinline__ float gate(float d) { return fmaxf(kGateBase, kGateRe
 
 __device__ __forceinline__ bool inside(int x, int y, int w, int h) { return x >= 0 && x < w && y >= 0 && y < h; }
 
-__global__ void pack_input_kernel(const float* __restrict__ depth, float4* __restrict__ X, int batch, int w, int h) {
-  const long long n = static_cast<long long>(batch) * w * h;
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int x = static_cast<int>(i % w), y = static_cast<int>((i / w) % h);
-    const long long img = i / (static_cast<long long>(w) * h);
-    const float d = depth[i];
-    float sum = 0.0f;
-    int cnt = 0;
-    for (int dy = -1; dy <= 1; ++dy) {
-      for (int dx = -1; dx <= 1; ++dx) {
-        if (!inside(x + dx, y + dy, w, h)) continue;
-        const float v = depth[(img * h + y + dy) * w + x + dx];
-        if (v > 0.0f) {
-          sum += v;
+// ---- packed single-precision arithmetic: two FP32 multiply-adds per instruction ----
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// two BF16 of one word as FP32
+__device__ __forceinline__ f32x2 bf2_to_f32x2(uint32_t v) {
+  return pack2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
+}
+
+// The tiles of the CUDA-core layers: kTileW x kTileH pixels of one image, 256 threads, warp w on rows w and w + 8
+// (thread: pixels (lane, w) and (lane, w + 8)).
+constexpr int kTileW = 32, kTileH = 16, kTileThreads = 256;
+
+struct TileGrid {
+  int tx, ty;
+  long long count;
+};
+__host__ __device__ inline TileGrid tile_grid(int batch, int w, int h, int tw, int th) {
+  TileGrid g{(w + tw - 1) / tw, (h + th - 1) / th, 0};
+  g.count = static_cast<long long>(batch) * g.tx * g.ty;
+  return g;
+}
+__device__ __forceinline__ void tile_at(const TileGrid& g, long long t, int tw, int th, int& img, int& x0, int& y0) {
+  const uint32_t i = static_cast<uint32_t>(t), row = i / static_cast<uint32_t>(g.tx);
+  x0 = static_cast<int>(i - row * static_cast<uint32_t>(g.tx)) * tw;
+  img = static_cast<int>(row / static_cast<uint32_t>(g.ty));
+  y0 = static_cast<int>(row - static_cast<uint32_t>(img) * static_cast<uint32_t>(g.ty)) * th;
+}
+
+// The input channels (see above) of the tile at (x0, y0) and a ring of one pixel around it, from the depth, staged
+// with a ring of two (0 outside the image, which counts as invalid).
+template <int TW, int TH>
+struct InputTile {
+  float depth[TH + 4][TW + 4];
+  float4 X[TH + 2][TW + 2];
+};
+// the depth words of a tile that a thread stages, in flight while the tile before is worked on
+template <int TW, int TH>
+struct DepthAhead {
+  static constexpr int kPer = ((TH + 4) * (TW + 4) + kTileThreads - 1) / kTileThreads;
+  float v[kPer];
+  __device__ __forceinline__ void load(const float* __restrict__ depth, int img, int x0, int y0, int w, int h) {
+    const float* d0 = depth + static_cast<size_t>(img) * w * h;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      const int i = threadIdx.x + k * kTileThreads, r = i / (TW + 4), c = i - r * (TW + 4);
+      const int x = x0 + c - 2, y = y0 + r - 2;
+      v[k] = r < TH + 4 && inside(x, y, w, h) ? __ldg(d0 + static_cast<size_t>(y) * w + x) : 0.0f;
+    }
+  }
+};
+template <int TW, int TH>
+__device__ __forceinline__ void stage_input(InputTile<TW, TH>& S, const DepthAhead<TW, TH>& ahead) {
+#pragma unroll
+  for (int k = 0; k < DepthAhead<TW, TH>::kPer; ++k) {
+    const int i = threadIdx.x + k * kTileThreads;
+    if (i < (TH + 4) * (TW + 4)) (&S.depth[0][0])[i] = ahead.v[k];
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < (TH + 2) * (TW + 2); i += kTileThreads) {
+    const int r = i / (TW + 2), c = i - r * (TW + 2);
+    const float d = S.depth[r + 1][c + 1];
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (d > 0.0f) {
+      float sum = 0.0f;
+      int cnt = 0;
+#pragma unroll
+      for (int t = 0; t < 9; ++t) {
+        const float n = S.depth[r + t / 3][c + t % 3];
+        if (n > 0.0f) {
+          sum += n;
           ++cnt;
         }
       }
+      const float m = sum / static_cast<float>(cnt);  // at least the pixel itself
+      v = make_float4((d - m) * kScale, 1.0f, m * 0.25f, 0.0f);
     }
-    const bool valid = d > 0.0f;
-    const float m = cnt ? sum / static_cast<float>(cnt) : 0.0f;
-    X[i] = valid ? make_float4((d - m) * kScale, 1.0f, m * 0.25f, 0.0f) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    S.X[r][c] = v;
   }
+  __syncthreads();
 }
 
-// layer 1: 4 -> 32, ReLU, one thread per pixel; weights staged tap-major as float4 over the 4 input channels
-// (sw4[t][co] = w1[co][0..3][t]) so that one 16-byte shared load feeds 4 multiply-adds.  The 9 taps' loads
-// are issued together, and each warp writes its 32 pixels x 64 bytes through its shared-memory buffer
-// (epi_pos), 512 contiguous bytes per store instruction; the loop runs over whole warps so that every lane
-// takes part in the buffer's warp-synchronous steps.
-__global__ void __launch_bounds__(256) conv_in_kernel(const float4* __restrict__ X, const float* __restrict__ params,
-                                                      __nv_bfloat16* __restrict__ A1, int batch, int w, int h) {
-  __shared__ float4 sw4[9][kC];
-  __shared__ float sb[kC];
-  __shared__ uint4 sbuf[8][128];  // one 2 KB transpose buffer per warp of the 256 threads
-  for (int i = threadIdx.x; i < 9 * kC; i += blockDim.x) {
-    const int t = i / kC, co = i % kC;
-    const float* wc = params + kOffW1 + co * kCin * 9;
-    sw4[t][co] = make_float4(wc[0 * 9 + t], wc[1 * 9 + t], wc[2 * 9 + t], wc[3 * 9 + t]);
+// a warp's 32 pixels of row y from (x0, y), 64 bytes each, between a lane per pixel and global memory through its
+// shared-memory buffer (epi_pos): 512 contiguous bytes per access instruction
+__device__ __forceinline__ void store_row32(uint4* buf, const uint4 (&v)[4], __nv_bfloat16* __restrict__ out, size_t row,
+                                            int x0, int w, int lane) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) buf[epi_pos(lane, q)] = v[q];
+  __syncwarp();
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int p = 8 * u + (lane >> 2), q = lane & 3;
+    if (x0 + p < w) *reinterpret_cast<uint4*>(out + (row + x0 + p) * kC + 8 * q) = buf[epi_pos(p, q)];
   }
-  for (int i = threadIdx.x; i < kC; i += blockDim.x) sb[i] = params[kOffB1 + i];
-  __syncthreads();
-  const long long n = static_cast<long long>(batch) * w * h;
+  __syncwarp();
+}
+// The 32 pixels from (x0, row) copied into a warp's buffer without passing through registers (0 outside the image),
+// pixel p's chunk q at epi_pos(p, q) or, kLinear, at 4 p + q: read by the same warp once async_wait has passed.
+template <bool kLinear>
+__device__ __forceinline__ void async_row32(uint4* buf, const __nv_bfloat16* __restrict__ in, size_t row, int x0, int w,
+                                            bool row_in, int lane) {
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int p = 8 * u + (lane >> 2), q = lane & 3, x = x0 + p;
+    const bool ok = row_in && x >= 0 && x < w;
+    const __nv_bfloat16* src = ok ? in + (row + x) * kC + 8 * q : in;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(&buf[kLinear ? 4 * p + q : epi_pos(p, q)])),
+                 "l"(src), "r"(ok ? 16 : 0)
+                 : "memory");
+  }
+}
+__device__ __forceinline__ void async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+// all but the newest kAhead groups of this thread have arrived; the warp's lanes see each other's
+template <int kAhead>
+__device__ __forceinline__ void async_wait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(kAhead) : "memory");
+  __syncwarp();
+}
+
+// layer 1: the input channels from the depth (in shared memory only), 4 -> 32, ReLU; the fourth channel is always 0 and
+// takes no products.  Two pixels per thread share the weights' shared-memory reads, and two output channels go
+// through one packed multiply-add: 27 x 16 of them a pixel.  Bound by FP32 arithmetic (105 us at the full rate for a batch
+// of 16 640x480 frames): 260 us, against 457 with the channels in global memory, one pixel a thread and scalar
+// multiply-adds; the next tile's depth is loaded during this one's products (283 us without).
+__global__ void __launch_bounds__(kTileThreads, 2) conv_in_kernel(const float* __restrict__ depth,
+                                                                  const float* __restrict__ params,
+                                                                  __nv_bfloat16* __restrict__ A1, int batch, int w, int h) {
+  __shared__ InputTile<kTileW, kTileH> S;
+  __shared__ __align__(16) float sw[9][3][kC];
+  __shared__ __align__(16) float sb[kC];
+  __shared__ uint4 sbuf[kTileThreads / 32][128];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint4* buf = sbuf[warp];
-  const long long warps = static_cast<long long>(gridDim.x) * (blockDim.x >> 5);
-  for (long long base = (blockIdx.x * static_cast<long long>(blockDim.x >> 5) + warp) * 32; base < n;
-       base += warps * 32) {
-    const long long i = base + lane;
-    float4 in[9];
-    if (i < n) {
-      // 32-bit coordinates (the launcher keeps the pixel count below 2^31)
-      const uint32_t i32 = static_cast<uint32_t>(i), row = i32 / static_cast<uint32_t>(w);
-      const int x = static_cast<int>(i32 - row * static_cast<uint32_t>(w));
-      const uint32_t im = row / static_cast<uint32_t>(h);
-      const int y = static_cast<int>(row - im * static_cast<uint32_t>(h));
-      const long long img = im;
-#pragma unroll
-      for (int t = 0; t < 9; ++t) {
-        const int sx = x + t % 3 - 1, sy = y + t / 3 - 1;
-        in[t] = inside(sx, sy, w, h) ? X[(img * h + sy) * w + sx] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      }
-    } else {
-#pragma unroll
-      for (int t = 0; t < 9; ++t) in[t] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  for (int i = threadIdx.x; i < 9 * 3 * kC; i += kTileThreads) {
+    const int t = i / (3 * kC), ci = (i / kC) % 3, co = i % kC;
+    sw[t][ci][co] = params[kOffW1 + (co * kCin + ci) * 9 + t];
+  }
+  if (threadIdx.x < kC) sb[threadIdx.x] = params[kOffB1 + threadIdx.x];
+  const TileGrid g = tile_grid(batch, w, h, kTileW, kTileH);
+  int img, x0, y0;
+  DepthAhead<kTileW, kTileH> ahead;
+  if (blockIdx.x < g.count) {
+    tile_at(g, blockIdx.x, kTileW, kTileH, img, x0, y0);
+    ahead.load(depth, img, x0, y0, w, h);
+  }
+  for (long long tile = blockIdx.x; tile < g.count; tile += gridDim.x) {
+    tile_at(g, tile, kTileW, kTileH, img, x0, y0);
+    __syncthreads();  // the previous tile has been read
+    stage_input(S, ahead);
+    if (tile + gridDim.x < g.count) {
+      int nimg, nx0, ny0;
+      tile_at(g, tile + gridDim.x, kTileW, kTileH, nimg, nx0, ny0);
+      ahead.load(depth, nimg, nx0, ny0, w, h);
     }
-    float acc[kC];
+    f32x2 acc[2][kC / 2];
 #pragma unroll
-    for (int co = 0; co < kC; ++co) acc[co] = sb[co];
-#pragma unroll
+    for (int c = 0; c < kC / 2; ++c) acc[0][c] = acc[1][c] = reinterpret_cast<const f32x2*>(sb)[c];
+#pragma unroll 1
     for (int t = 0; t < 9; ++t) {
+      const float4 xa = S.X[warp + t / 3][lane + t % 3], xb = S.X[warp + 8 + t / 3][lane + t % 3];
+      const float va[3] = {xa.x, xa.y, xa.z}, vb[3] = {xb.x, xb.y, xb.z};
 #pragma unroll
-      for (int co = 0; co < kC; ++co) {
-        const float4 wv = sw4[t][co];
-        acc[co] += wv.x * in[t].x + wv.y * in[t].y + wv.z * in[t].z + wv.w * in[t].w;
+      for (int ci = 0; ci < 3; ++ci) {
+        const f32x2 pa = pack2(va[ci], va[ci]), pb = pack2(vb[ci], vb[ci]);
+        const ulonglong2* wp = reinterpret_cast<const ulonglong2*>(sw[t][ci]);
+#pragma unroll
+        for (int c = 0; c < kC / 4; ++c) {
+          const ulonglong2 wv = wp[c];
+          acc[0][2 * c] = fma2(wv.x, pa, acc[0][2 * c]);
+          acc[0][2 * c + 1] = fma2(wv.y, pa, acc[0][2 * c + 1]);
+          acc[1][2 * c] = fma2(wv.x, pb, acc[1][2 * c]);
+          acc[1][2 * c + 1] = fma2(wv.y, pb, acc[1][2 * c + 1]);
+        }
       }
     }
-    __align__(16) __nv_bfloat162 res[kC / 2];
 #pragma unroll
-    for (int c = 0; c < kC / 2; ++c) res[c] = __floats2bfloat162_rn(fmaxf(acc[2 * c], 0.0f), fmaxf(acc[2 * c + 1], 0.0f));
+    for (int r = 0; r < 2; ++r) {
+      const int y = y0 + warp + 8 * r;
+      __align__(16) __nv_bfloat162 res[kC / 2];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) buf[epi_pos(lane, q)] = reinterpret_cast<const uint4*>(res)[q];
+      for (int c = 0; c < kC / 2; ++c) {
+        float lo, hi;
+        unpack2(acc[r][c], lo, hi);
+        res[c] = __floats2bfloat162_rn(fmaxf(lo, 0.0f), fmaxf(hi, 0.0f));
+      }
+      uint4 v[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) v[q] = reinterpret_cast<const uint4*>(res)[q];
+      if (y < h) store_row32(sbuf[warp], v, A1, (static_cast<size_t>(img) * h + y) * w, x0, w, lane);
+    }
+  }
+}
+
+// layer 4: 32 -> 1 residual, depth' = d + r / 100 on valid pixels.  Every input pixel's products with the 9 taps'
+// weights are summed over its channels once (9 sums a pixel, packed multiply-adds over channel pairs, two pixels a
+// thread sharing the weights' reads) and an output pixel adds 9 of those sums from shared memory; a CTA's 32 x 16
+// input pixels give 30 x 14 outputs.  148 us for a batch of 16 640x480 frames; one thread per (output pixel, 8
+// channels) read and converted every activation 9 times: 380 us.
+constexpr int kOutW = kTileW - 2, kOutH = kTileH - 2, kOutCtas = 3;
+constexpr int kOutRowBytes = kTileThreads / 32 * 2 * 128 * 16, kOutSmem = kOutRowBytes + 9 * kTileH * kTileW * 4;
+
+__global__ void __launch_bounds__(kTileThreads, kOutCtas) conv_out_kernel(const __nv_bfloat16* __restrict__ A3,
+                                                                   const float* __restrict__ params,
+                                                                   const float* __restrict__ depth,
+                                                                   const float* __restrict__ fallback,
+                                                                   float* __restrict__ out, int batch, int w, int h) {
+  extern __shared__ __align__(16) unsigned char out_smem[];
+  uint4(*rows)[2][128] = reinterpret_cast<uint4(*)[2][128]>(out_smem);  // [warp][row][chunk]
+  float(*S)[kTileH][kTileW] = reinterpret_cast<float(*)[kTileH][kTileW]>(out_smem + kOutRowBytes);
+  __shared__ __align__(16) float sw[9][kC];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int i = threadIdx.x; i < 9 * kC; i += kTileThreads) sw[i / kC][i % kC] = params[kOffW4 + (i % kC) * 9 + i / kC];
+  const float sb = params[kOffB4];
+  const TileGrid g = tile_grid(batch, w, h, kOutW, kOutH);
+  auto fetch = [&](long long tile) {  // this warp's two rows of a tile, in flight while the tile before is worked on
+    if (tile < g.count) {
+      int img, x0, y0;
+      tile_at(g, tile, kOutW, kOutH, img, x0, y0);
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const int y = y0 - 1 + warp + 8 * r;
+        const bool in = y >= 0 && y < h;
+        async_row32<false>(rows[warp][r], A3, (static_cast<size_t>(img) * h + (in ? y : 0)) * w, x0 - 1, w, in, lane);
+      }
+    }
+    async_commit();
+  };
+  fetch(blockIdx.x);
+  for (long long tile = blockIdx.x; tile < g.count; tile += gridDim.x) {
+    int img, x0, y0;
+    tile_at(g, tile, kOutW, kOutH, img, x0, y0);
+    const size_t base = static_cast<size_t>(img) * h;
+    uint4 a[2][4];
+    async_wait<0>();
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) a[r][q] = rows[warp][r][epi_pos(lane, q)];
+    }
     __syncwarp();
+    fetch(tile + gridDim.x);
+    __syncthreads();  // the weights; the previous tile's sums have been read
+    f32x2 acc[2][9];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int p = 8 * u + (lane >> 2), q = lane & 3;
-      if (base + p < n) *reinterpret_cast<uint4*>(A1 + (base + p) * kC + 8 * q) = buf[epi_pos(p, q)];
-    }
-    __syncwarp();  // the buffer is rewritten by the next group
-  }
-}
-
-__device__ __forceinline__ void load32(const __nv_bfloat16* p, float* v) {
-  __align__(16) __nv_bfloat16 b[kC];
+    for (int t = 0; t < 9; ++t) acc[0][t] = acc[1][t] = 0ULL;
 #pragma unroll
-  for (int q = 0; q < 4; ++q) reinterpret_cast<uint4*>(b)[q] = reinterpret_cast<const uint4*>(p)[q];
+    for (int q = 0; q < 4; ++q) {
+      const uint32_t w0[4] = {a[0][q].x, a[0][q].y, a[0][q].z, a[0][q].w};
+      const uint32_t w1[4] = {a[1][q].x, a[1][q].y, a[1][q].z, a[1][q].w};
 #pragma unroll
-  for (int c = 0; c < kC; ++c) v[c] = __bfloat162float(b[c]);
-}
-
-// layer 4: 32 -> 1 residual, depth' = d + r / 100 on valid pixels; weights staged tap-major (sw[t][c]) and
-// read as float4.  Four lanes per pixel, lane q = lane % 4 summing channels 8q..8q+7 over the taps: a warp
-// covers 8 consecutive pixels, so its 16-byte loads of their 64-byte channel vectors are contiguous, and the
-// 9 taps' loads are issued together.  The pixel's four lanes then add their sums; the loop runs over
-// warp-sized groups of 8 pixels so that every lane takes part in the shuffles.
-__global__ void __launch_bounds__(256) conv_out_kernel(const __nv_bfloat16* __restrict__ A3,
-                                                       const float* __restrict__ params,
-                                                       const float* __restrict__ depth,
-                                                       const float* __restrict__ fallback, float* __restrict__ out,
-                                                       int batch, int w, int h) {
-  __shared__ float4 sw4[9][kC / 4];
-  __shared__ float sb;
-  for (int i = threadIdx.x; i < 9 * kC; i += blockDim.x) {
-    const int t = i / kC, c = i % kC;
-    reinterpret_cast<float*>(&sw4[t][0])[c] = params[kOffW4 + c * 9 + t];
-  }
-  if (threadIdx.x == 0) sb = params[kOffB4];
-  __syncthreads();
-  const long long n = static_cast<long long>(batch) * w * h;
-  const int lane = threadIdx.x & 31, q = lane & 3;
-  const long long warps = static_cast<long long>(gridDim.x) * (blockDim.x >> 5);
-  for (long long base = (blockIdx.x * static_cast<long long>(blockDim.x >> 5) + (threadIdx.x >> 5)) * 8; base < n;
-       base += warps * 8) {
-    const long long i = base + (lane >> 2);
-    const float d = i < n ? depth[i] : 0.0f;
-    float r = 0.0f;
-    if (d > 0.0f) {
-      const uint32_t i32 = static_cast<uint32_t>(i), row = i32 / static_cast<uint32_t>(w);  // 32-bit, as in conv_in
-      const int x = static_cast<int>(i32 - row * static_cast<uint32_t>(w));
-      const uint32_t im = row / static_cast<uint32_t>(h);
-      const int y = static_cast<int>(row - im * static_cast<uint32_t>(h));
-      const long long img = im;
-      // the 9 taps' loads are issued together (zero outside the image, which adds nothing), then used
-      uint4 raw9[9];
+      for (int j = 0; j < 2; ++j) {
+        const f32x2 p0 = bf2_to_f32x2(w0[2 * j]), p1 = bf2_to_f32x2(w0[2 * j + 1]);
+        const f32x2 r0 = bf2_to_f32x2(w1[2 * j]), r1 = bf2_to_f32x2(w1[2 * j + 1]);
 #pragma unroll
-      for (int t = 0; t < 9; ++t) {
-        const int sx = x + t % 3 - 1, sy = y + t / 3 - 1;
-        raw9[t] = inside(sx, sy, w, h) ? *reinterpret_cast<const uint4*>(A3 + ((img * h + sy) * w + sx) * kC + 8 * q)
-                                       : make_uint4(0, 0, 0, 0);
-      }
-#pragma unroll
-      for (int t = 0; t < 9; ++t) {
-        const __nv_bfloat162* b2 = reinterpret_cast<const __nv_bfloat162*>(&raw9[t]);
-        const float4 wa = sw4[t][2 * q], wb = sw4[t][2 * q + 1];
-        const float2 a0 = __bfloat1622float2(b2[0]), a1 = __bfloat1622float2(b2[1]);
-        const float2 a2 = __bfloat1622float2(b2[2]), a3 = __bfloat1622float2(b2[3]);
-        r += wa.x * a0.x + wa.y * a0.y + wa.z * a1.x + wa.w * a1.y + wb.x * a2.x + wb.y * a2.y + wb.z * a3.x +
-             wb.w * a3.y;
+        for (int t = 0; t < 9; ++t) {
+          const ulonglong2 wv = *reinterpret_cast<const ulonglong2*>(&sw[t][8 * q + 4 * j]);
+          acc[0][t] = fma2(wv.y, p1, fma2(wv.x, p0, acc[0][t]));
+          acc[1][t] = fma2(wv.y, r1, fma2(wv.x, r0, acc[1][t]));
+        }
       }
     }
-    r += __shfl_xor_sync(0xffffffffU, r, 1);
-    r += __shfl_xor_sync(0xffffffffU, r, 2);
-    if (q == 0 && i < n) {
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+#pragma unroll
+      for (int t = 0; t < 9; ++t) {
+        float lo, hi;
+        unpack2(acc[r][t], lo, hi);
+        S[t][warp + 8 * r][lane] = lo + hi;
+      }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < kOutW * kOutH; i += kTileThreads) {
+      const int oy = i / kOutW, ox = i - oy * kOutW;
+      const int x = x0 + ox, y = y0 + oy;
+      if (x >= w || y >= h) continue;
+      const size_t at = (base + y) * w + x;
+      const float d = depth[at];
       if (!(d > 0.0f)) {
-        out[i] = 0.0f;
-      } else {
-        const float corr = (sb + r) * kInvScale;
-        out[i] = (fallback && fabsf(corr) > gate(d)) ? fallback[i] : fmaxf(d + corr, 0.0f);
+        out[at] = 0.0f;
+        continue;
       }
+      float r = 0.0f;
+#pragma unroll
+      for (int t = 0; t < 9; ++t) r += S[t][oy + t / 3][ox + t % 3];
+      const float corr = (sb + r) * kInvScale;
+      out[at] = (fallback && fabsf(corr) > gate(d)) ? fallback[at] : fmaxf(d + corr, 0.0f);
     }
   }
 }
 
-// loss = sum over pixels valid in input, target and output whose input and target agree within the
-// discontinuity threshold, of (out - target)^2 / n_pixels; dr = dloss/dr
-__global__ void loss_grad_kernel(const float* __restrict__ out, const float* __restrict__ target,
-                                 const float* __restrict__ depth, float* __restrict__ dr, long long n,
-                                 float* __restrict__ loss) {
-  float se = 0.0f, cnt = 0.0f;
-  const float inv_n = 1.0f / static_cast<float>(n);
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const bool m = depth[i] > 0.0f && target[i] > 0.0f && out[i] > 0.0f && fabsf(depth[i] - target[i]) <= gate(target[i]);
-    const float diff = m ? out[i] - target[i] : 0.0f;
-    dr[i] = 2.0f * diff * kInvScale * inv_n;
-    se += diff * diff;
-    cnt += m ? 1.0f : 0.0f;
+// The output layer's backward pass in one read of the activations A3:
+//   the loss (sum over pixels valid in input, target and output whose input and target agree within the discontinuity
+//   threshold, of (out - target)^2 / n_pixels) and dr = dloss/dr of the tile and a ring around it, in shared memory;
+//   dA3[q][c] = (A3[q][c] > 0) * sum_t w4[c][t] dr[q - off(t)], BF16 (packed multiply-adds over channel pairs, two
+//   pixels a thread);
+//   dw4[c][t] += sum_q A3[q][c] dr[q - off(t)], db4 += sum_q dr[q]: lane = (channel pair, half of the warp's 32
+//   pixels), the 9 taps' dr sliding along the row in registers; summed over the CTA's tiles, one atomic per weight.
+// 283 us for a batch of 16 640x480 frames (HBM needs 92, FP32 arithmetic 70); as three kernels, the weight gradients
+// from segments staged three rows at a time, 723 us.
+constexpr int kOutBackSmem = 2 * kTileThreads / 32 * 2 * 128 * 16;  // two stages of a tile's activations
+
+__global__ void __launch_bounds__(kTileThreads, 2) out_backward_kernel(
+    const __nv_bfloat16* __restrict__ A3, const float* __restrict__ params, const float* __restrict__ depth,
+    const float* __restrict__ target, const float* __restrict__ out, __nv_bfloat16* __restrict__ dA3,
+    float* __restrict__ dw4, float* __restrict__ db4, float* __restrict__ loss, int batch, int w, int h) {
+  constexpr int kWarps = kTileThreads / 32, kRing = (kTileH + 2) * (kTileW + 2);
+  constexpr int kPer = (kRing + kTileThreads - 1) / kTileThreads;
+  extern __shared__ __align__(16) unsigned char out_smem[];
+  uint4(*rows)[kWarps][2][128] = reinterpret_cast<uint4(*)[kWarps][2][128]>(out_smem);  // [stage][warp][row][chunk]
+  __shared__ __align__(16) float sw[9][kC];
+  __shared__ float sdr[kTileH + 2][kTileW + 2];
+  __shared__ uint4 sbuf[kWarps][128];
+  __shared__ float sred[9][kC];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int i = threadIdx.x; i < 9 * kC; i += kTileThreads) {
+    sw[i / kC][i % kC] = params[kOffW4 + (i % kC) * 9 + i / kC];
+    sred[i / kC][i % kC] = 0.0f;
+  }
+  const float inv_n = 1.0f / static_cast<float>(static_cast<long long>(batch) * w * h);
+  const int pair = lane & 15, part = lane >> 4;
+  f32x2 wacc[9];
+#pragma unroll
+  for (int t = 0; t < 9; ++t) wacc[t] = 0ULL;
+  float se = 0.0f, cnt = 0.0f, dsum = 0.0f;
+  const TileGrid g = tile_grid(batch, w, h, kTileW, kTileH);
+  // a tile's activations (this warp's two rows) and the depth, target and output of its ring: in flight while the
+  // tile before is worked on
+  float fd[kPer], ft[kPer], fo[kPer];
+  auto fetch = [&](long long tile, int stage) {
+    if (tile < g.count) {
+      int img, x0, y0;
+      tile_at(g, tile, kTileW, kTileH, img, x0, y0);
+      const size_t base = static_cast<size_t>(img) * h;
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const int y = y0 + warp + 8 * r;
+        async_row32<false>(rows[stage][warp][r], A3, (base + min(y, h - 1)) * w, x0, w, y < h, lane);
+      }
+#pragma unroll
+      for (int k = 0; k < kPer; ++k) {
+        const int i = threadIdx.x + k * kTileThreads, r = i / (kTileW + 2), c = i - r * (kTileW + 2);
+        const int x = x0 + c - 1, y = y0 + r - 1;
+        fd[k] = ft[k] = fo[k] = 0.0f;
+        if (i < kRing && inside(x, y, w, h)) {
+          const size_t at = (base + y) * w + x;
+          fd[k] = __ldg(depth + at);
+          ft[k] = __ldg(target + at);
+          fo[k] = __ldg(out + at);
+        }
+      }
+    }
+    async_commit();
+  };
+  fetch(blockIdx.x, 0);
+  int stage = 0;
+  for (long long tile = blockIdx.x; tile < g.count; tile += gridDim.x, stage ^= 1) {
+    int img, x0, y0;
+    tile_at(g, tile, kTileW, kTileH, img, x0, y0);
+    const size_t base = static_cast<size_t>(img) * h;
+    __syncthreads();  // the previous tile's dr has been read
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      const int i = threadIdx.x + k * kTileThreads, r = i / (kTileW + 2), c = i - r * (kTileW + 2);
+      if (i >= kRing) break;
+      const float d = fd[k], t = ft[k], o = fo[k];  // 0 outside the image
+      const bool m = d > 0.0f && t > 0.0f && o > 0.0f && fabsf(d - t) <= gate(t);
+      const float diff = m ? o - t : 0.0f;
+      const float v = 2.0f * diff * kInvScale * inv_n;
+      if (r >= 1 && r <= kTileH && c >= 1 && c <= kTileW) {
+        se += diff * diff;
+        cnt += m ? 1.0f : 0.0f;
+        dsum += v;
+      }
+      sdr[r][c] = v;
+    }
+    __syncthreads();
+    fetch(tile + gridDim.x, stage ^ 1);
+    async_wait<1>();
+    const uint4(*act)[128] = rows[stage][warp];
+    // the activations' gradient
+    f32x2 acc[2][kC / 2];
+#pragma unroll
+    for (int c = 0; c < kC / 2; ++c) acc[0][c] = acc[1][c] = 0ULL;
+#pragma unroll 1
+    for (int t = 0; t < 9; ++t) {
+      const float ga = sdr[warp + 2 - t / 3][lane + 2 - t % 3], gb = sdr[warp + 10 - t / 3][lane + 2 - t % 3];
+      const f32x2 pa = pack2(ga, ga), pb = pack2(gb, gb);
+      const ulonglong2* wp = reinterpret_cast<const ulonglong2*>(sw[t]);
+#pragma unroll
+      for (int c = 0; c < kC / 4; ++c) {
+        const ulonglong2 wv = wp[c];
+        acc[0][2 * c] = fma2(wv.x, pa, acc[0][2 * c]);
+        acc[0][2 * c + 1] = fma2(wv.y, pa, acc[0][2 * c + 1]);
+        acc[1][2 * c] = fma2(wv.x, pb, acc[1][2 * c]);
+        acc[1][2 * c + 1] = fma2(wv.y, pb, acc[1][2 * c + 1]);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const int y = y0 + warp + 8 * r;
+      __align__(16) __nv_bfloat162 res[kC / 2];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const uint4 a4 = act[r][epi_pos(lane, q)];
+        const uint32_t words[4] = {a4.x, a4.y, a4.z, a4.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          float lo, hi, alo, ahi;
+          unpack2(acc[r][4 * q + j], lo, hi);
+          unpack2(bf2_to_f32x2(words[j]), alo, ahi);
+          res[4 * q + j] = __floats2bfloat162_rn(alo > 0.0f ? lo : 0.0f, ahi > 0.0f ? hi : 0.0f);
+        }
+      }
+      uint4 v[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) v[q] = reinterpret_cast<const uint4*>(res)[q];
+      if (y < h) store_row32(sbuf[warp], v, dA3, (base + y) * w, x0, w, lane);
+    }
+    // the weights' gradients: word `pair` of pixel p is in its chunk pair / 4
+#pragma unroll 1
+    for (int r = 0; r < 2; ++r) {
+      const uint32_t* words = reinterpret_cast<const uint32_t*>(act[r]);
+      const int row = warp + 8 * r, p0 = 16 * part;
+      // dr at column p + 2 - kx of rows row + 2 - ky: the window's columns p (kx = 2), p + 1, p + 2 (kx = 0)
+      f32x2 win[3][3];  // [ky][column]
+#pragma unroll
+      for (int ky = 0; ky < 3; ++ky) {
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const float v = sdr[row + 2 - ky][p0 + c];
+          win[ky][c + 1] = pack2(v, v);
+        }
+      }
+#pragma unroll 4
+      for (int p = p0; p < p0 + 16; ++p) {
+#pragma unroll
+        for (int ky = 0; ky < 3; ++ky) {
+          const float v = sdr[row + 2 - ky][p + 2];
+          win[ky][0] = win[ky][1];
+          win[ky][1] = win[ky][2];
+          win[ky][2] = pack2(v, v);
+        }
+        const f32x2 av = bf2_to_f32x2(words[4 * epi_pos(p, pair >> 2) + (pair & 3)]);
+#pragma unroll
+        for (int ky = 0; ky < 3; ++ky) {
+#pragma unroll
+          for (int kx = 0; kx < 3; ++kx) wacc[3 * ky + kx] = fma2(av, win[ky][2 - kx], wacc[3 * ky + kx]);
+        }
+      }
+    }
+    __syncwarp();  // the stage is refilled after the next tile's start
+  }
+  __syncthreads();
+#pragma unroll
+  for (int t = 0; t < 9; ++t) {
+    float lo, hi;
+    unpack2(wacc[t], lo, hi);
+    lo += __shfl_xor_sync(0xffffffffu, lo, 16);
+    hi += __shfl_xor_sync(0xffffffffu, hi, 16);
+    if (part == 0) {
+      atomicAdd(&sred[t][2 * pair], lo);
+      atomicAdd(&sred[t][2 * pair + 1], hi);
+    }
   }
   for (int o = 16; o > 0; o >>= 1) {
-    se += __shfl_down_sync(0xffffffffU, se, o);
-    cnt += __shfl_down_sync(0xffffffffU, cnt, o);
+    se += __shfl_down_sync(0xffffffffu, se, o);
+    cnt += __shfl_down_sync(0xffffffffu, cnt, o);
+    dsum += __shfl_down_sync(0xffffffffu, dsum, o);
   }
-  if ((threadIdx.x & 31) == 0) {
+  if (lane == 0) {
     atomicAdd(&loss[0], se);
     atomicAdd(&loss[1], cnt);
+    atomicAdd(db4, dsum);
   }
-}
-
-// dA3[q][c] = (A3[q][c] > 0) * sum_t w4[c][t] dr[q - off(t)]
-__global__ void __launch_bounds__(256) dgrad_out_kernel(const float* __restrict__ dr, const float* __restrict__ params,
-                                                        const __nv_bfloat16* __restrict__ A3,
-                                                        __nv_bfloat16* __restrict__ dA3, int batch, int w, int h) {
-  __shared__ float sw[kC * 9];
-  for (int i = threadIdx.x; i < kC * 9; i += blockDim.x) sw[i] = params[kOffW4 + i];
   __syncthreads();
-  const long long n = static_cast<long long>(batch) * w * h;
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int x = static_cast<int>(i % w), y = static_cast<int>((i / w) % h);
-    const long long img = i / (static_cast<long long>(w) * h);
-    float g[9];
-#pragma unroll
-    for (int t = 0; t < 9; ++t) {
-      const int sx = x - (t % 3 - 1), sy = y - (t / 3 - 1);
-      g[t] = inside(sx, sy, w, h) ? dr[(img * h + sy) * w + sx] : 0.0f;
-    }
-    float a[kC];
-    load32(A3 + i * kC, a);
-    __align__(16) __nv_bfloat16 res[kC];
-#pragma unroll
-    for (int c = 0; c < kC; ++c) {
-      float acc = 0.0f;
-#pragma unroll
-      for (int t = 0; t < 9; ++t) acc += sw[c * 9 + t] * g[t];
-      res[c] = __float2bfloat16_rn(a[c] > 0.0f ? acc : 0.0f);
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) reinterpret_cast<uint4*>(dA3 + i * kC)[q] = reinterpret_cast<const uint4*>(res)[q];
-  }
+  for (int i = threadIdx.x; i < 9 * kC; i += kTileThreads) atomicAdd(&dw4[(i % kC) * 9 + i / kC], sred[i / kC][i % kC]);
 }
 
-// Weight gradients of the input and output layers (CUDA cores): dW[co][ci][t] = sum_p dY[p][co] X[p + off(t)][ci],
-// db[co] = sum_p dY[p][co].  X: BF16 with 32 channels (read as 16-byte vectors) or FP32 float4 (CI = 4); dY:
-// BF16 with 32 channels or FP32 with 1.  Each CTA stages row segments of kSeg pixels (three input rows with a
-// one-pixel halo, one gradient row) in shared memory as floats.  Thread (rep, co, ci) keeps 9 accumulators (and
-// the bias sum) over the rep-th of kRep contiguous runs of each segment, so that CI x CO x kRep threads share a
-// segment; the kRep partial sums are added in shared memory and flushed with one atomic per weight per CTA.
-constexpr int kSeg = 64;
+// The input layer's weight gradients dw1[co][ci][t] += sum_p dY[p][co] X[p + off(t)][ci], db1[co] += sum_p dY[p][co]:
+// lane = output channel, a warp runs along its row's 32 pixels with the 9 taps' input channels (from the depth, as in
+// conv_in_kernel) sliding in registers, two input channels per packed multiply-add; summed over the CTA's tiles, one
+// atomic per weight.  Bound by FP32 arithmetic and issue: 274 us for a batch of 16 640x480 frames, against 472 with
+// (output, input) channel threads over staged segments.
+constexpr int kWgInH = 8;  // rows of a tile: one per warp
 
-template <int CI, int CO, bool kXBf16, bool kDyBf16, int kRep>
-__global__ void __launch_bounds__(CI * CO * kRep) wgrad_kernel(const void* __restrict__ Xv, const void* __restrict__ dYv,
-                                                               float* __restrict__ dW, float* __restrict__ db,
-                                                               int batch, int w, int h) {
-  static_assert(!kXBf16 || CI == 32, "BF16 inputs carry 32 channels");
-  static_assert(kXBf16 || CI == 4, "FP32 inputs are float4 pixels");
-  static_assert(!kDyBf16 || CO == 32, "BF16 gradients carry 32 channels");
-  static_assert(kDyBf16 || CO == 1, "FP32 gradients carry one channel");
-  static_assert(kSeg % kRep == 0, "replicas take equal runs of a segment");
-  constexpr int kPairs = CI * CO, kT = kPairs * kRep;
-  __shared__ __align__(16) float sX[3][kSeg + 2][CI];
-  __shared__ __align__(16) float sG[kSeg][CO];
-  __shared__ float sRed[kRep > 1 ? kRep - 1 : 1][10][kPairs];
-  const int tid = threadIdx.x;
-  const int pair = tid % kPairs, rep = tid / kPairs;
-  const int co = pair / CI, ci = pair % CI;
-  float acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+__global__ void __launch_bounds__(kTileThreads, 2) wgrad_in_kernel(const float* __restrict__ depth,
+                                                                   const __nv_bfloat16* __restrict__ dY,
+                                                                   float* __restrict__ dw1, float* __restrict__ db1,
+                                                                   int batch, int w, int h) {
+  constexpr int kWarps = kTileThreads / 32;
+  static_assert(kWarps == kWgInH, "one row per warp");
+  __shared__ InputTile<kTileW, kWgInH> S;
+  __shared__ uint4 sbuf[2][kWarps][128];  // two stages of a row's gradients, 64 bytes a pixel
+  __shared__ float sred[kC * 3 * 9 + kC];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int i = threadIdx.x; i < kC * 3 * 9 + kC; i += kTileThreads) sred[i] = 0.0f;
+  f32x2 acc[9];   // channels 0 and 1
+  float acc2[9];  // channel 2
+#pragma unroll
+  for (int t = 0; t < 9; ++t) {
+    acc[t] = 0ULL;
+    acc2[t] = 0.0f;
+  }
   float bacc = 0.0f;
-  const int segs_x = (w + kSeg - 1) / kSeg;
-  const long long nseg = static_cast<long long>(batch) * h * segs_x;
-  for (long long sgi = blockIdx.x; sgi < nseg; sgi += gridDim.x) {
-    const int x0 = static_cast<int>(sgi % segs_x) * kSeg;
-    const int y = static_cast<int>((sgi / segs_x) % h);
-    const long long img = sgi / (static_cast<long long>(segs_x) * h);
-    if (kXBf16) {  // 4 vectors of 8 channels per pixel
-      for (int i = tid; i < 3 * (kSeg + 2) * 4; i += kT) {
-        const int q = i & 3, px = (i >> 2) % (kSeg + 2), r = (i >> 2) / (kSeg + 2);
-        const int sx = x0 - 1 + px, sy = y - 1 + r;
-        uint4 u = make_uint4(0u, 0u, 0u, 0u);
-        if (inside(sx, sy, w, h)) {
-          u = reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(Xv) + ((img * h + sy) * w + sx) * CI)[q];
+  const TileGrid g = tile_grid(batch, w, h, kTileW, kWgInH);
+  DepthAhead<kTileW, kWgInH> ahead;
+  auto fetch = [&](long long tile, int stage) {
+    if (tile < g.count) {
+      int img, x0, y0;
+      tile_at(g, tile, kTileW, kWgInH, img, x0, y0);
+      const int y = y0 + warp;
+      async_row32<true>(sbuf[stage][warp], dY, (static_cast<size_t>(img) * h + min(y, h - 1)) * w, x0, w, y < h, lane);
+      ahead.load(depth, img, x0, y0, w, h);
+    }
+    async_commit();
+  };
+  fetch(blockIdx.x, 0);
+  int stage = 0;
+  for (long long tile = blockIdx.x; tile < g.count; tile += gridDim.x, stage ^= 1) {
+    __syncthreads();  // the previous tile has been read
+    stage_input(S, ahead);
+    fetch(tile + gridDim.x, stage ^ 1);
+    async_wait<1>();
+    const uint16_t* gr = reinterpret_cast<const uint16_t*>(sbuf[stage][warp]);
+    f32x2 win[3][3];  // [ky][column]: a pixel's channels 0 and 1
+    float win2[3][3];  // channel 2
+    auto column = [&](int ky, int c, int to) {
+      const float4 v = S.X[warp + ky][c];
+      win[ky][to] = pack2(v.x, v.y);
+      win2[ky][to] = v.z;
+    };
+#pragma unroll
+    for (int ky = 0; ky < 3; ++ky) {
+      column(ky, 0, 1);
+      column(ky, 1, 2);
+    }
+#pragma unroll 3
+    for (int p = 0; p < kTileW; ++p) {
+      const float gv = __uint_as_float(static_cast<uint32_t>(gr[p * kC + lane]) << 16);
+      const f32x2 gp = pack2(gv, gv);
+#pragma unroll
+      for (int ky = 0; ky < 3; ++ky) {
+        win[ky][0] = win[ky][1];
+        win[ky][1] = win[ky][2];
+        win2[ky][0] = win2[ky][1];
+        win2[ky][1] = win2[ky][2];
+        column(ky, p + 2, 2);
+#pragma unroll
+        for (int kx = 0; kx < 3; ++kx) {
+          acc[3 * ky + kx] = fma2(gp, win[ky][kx], acc[3 * ky + kx]);
+          acc2[3 * ky + kx] = fmaf(gv, win2[ky][kx], acc2[3 * ky + kx]);
         }
-        const __nv_bfloat162* b2 = reinterpret_cast<const __nv_bfloat162*>(&u);
-        float4* dst = reinterpret_cast<float4*>(&sX[r][px][8 * q]);
-        const float2 f0 = __bfloat1622float2(b2[0]), f1 = __bfloat1622float2(b2[1]);
-        const float2 f2 = __bfloat1622float2(b2[2]), f3 = __bfloat1622float2(b2[3]);
-        dst[0] = make_float4(f0.x, f0.y, f1.x, f1.y);
-        dst[1] = make_float4(f2.x, f2.y, f3.x, f3.y);
       }
-    } else {  // one float4 per pixel
-      for (int i = tid; i < 3 * (kSeg + 2); i += kT) {
-        const int px = i % (kSeg + 2), r = i / (kSeg + 2);
-        const int sx = x0 - 1 + px, sy = y - 1 + r;
-        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (inside(sx, sy, w, h)) v = static_cast<const float4*>(Xv)[(img * h + sy) * w + sx];
-        *reinterpret_cast<float4*>(&sX[r][px][0]) = v;
-      }
+      bacc += gv;
     }
-    if (kDyBf16) {
-      for (int i = tid; i < kSeg * 4; i += kT) {
-        const int q = i & 3, px = i >> 2;
-        const int sx = x0 + px;
-        uint4 u = make_uint4(0u, 0u, 0u, 0u);
-        if (sx < w) u = reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(dYv) + ((img * h + y) * w + sx) * CO)[q];
-        const __nv_bfloat162* b2 = reinterpret_cast<const __nv_bfloat162*>(&u);
-        float4* dst = reinterpret_cast<float4*>(&sG[px][8 * q]);
-        const float2 f0 = __bfloat1622float2(b2[0]), f1 = __bfloat1622float2(b2[1]);
-        const float2 f2 = __bfloat1622float2(b2[2]), f3 = __bfloat1622float2(b2[3]);
-        dst[0] = make_float4(f0.x, f0.y, f1.x, f1.y);
-        dst[1] = make_float4(f2.x, f2.y, f3.x, f3.y);
-      }
-    } else {
-      for (int i = tid; i < kSeg; i += kT) {
-        const int sx = x0 + i;
-        sG[i][0] = sx < w ? static_cast<const float*>(dYv)[(img * h + y) * w + sx] : 0.0f;
-      }
-    }
-    __syncthreads();
-    // replica rep takes a contiguous run of the segment's pixels, so each tap row's three inputs slide along it:
-    // one new shared-memory read per row and pixel instead of three
-    constexpr int kRun = kSeg / kRep;
-    const int p0 = rep * kRun;
-    float w0[3], w1[3];
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-      w0[r] = sX[r][p0][ci];
-      w1[r] = sX[r][p0 + 1][ci];
-    }
-    for (int px = p0; px < p0 + kRun; ++px) {
-      const float g = sG[px][co];
-#pragma unroll
-      for (int r = 0; r < 3; ++r) {
-        const float w2 = sX[r][px + 2][ci];
-        acc[3 * r] += g * w0[r];
-        acc[3 * r + 1] += g * w1[r];
-        acc[3 * r + 2] += g * w2;
-        w0[r] = w1[r];
-        w1[r] = w2;
-      }
-      bacc += g;
-    }
-    __syncthreads();
+    __syncwarp();
   }
-  if (kRep > 1) {
-    if (rep > 0) {
+  __syncthreads();
 #pragma unroll
-      for (int t = 0; t < 9; ++t) sRed[rep - 1][t][pair] = acc[t];
-      sRed[rep - 1][9][pair] = bacc;
-    }
-    __syncthreads();
-    if (rep == 0) {
-      for (int r = 0; r < kRep - 1; ++r) {
+  for (int t = 0; t < 9; ++t) {
+    float v[3];
+    unpack2(acc[t], v[0], v[1]);
+    v[2] = acc2[t];
 #pragma unroll
-        for (int t = 0; t < 9; ++t) acc[t] += sRed[r][t][pair];
-        bacc += sRed[r][9][pair];
-      }
-    }
+    for (int ci = 0; ci < 3; ++ci) atomicAdd(&sred[(lane * 3 + ci) * 9 + t], v[ci]);
   }
-  if (rep == 0) {
-#pragma unroll
-    for (int t = 0; t < 9; ++t) atomicAdd(&dW[(co * CI + ci) * 9 + t], acc[t]);
-    if (ci == 0) atomicAdd(&db[co], bacc);
-  }
+  atomicAdd(&sred[kC * 3 * 9 + lane], bacc);
+  __syncthreads();
+  // [co][ci][t]; the gradients of the fourth channel, which is always 0, stay 0
+  for (int i = threadIdx.x; i < kC * 3 * 9; i += kTileThreads) atomicAdd(&dw1[i / 27 * (kCin * 9) + i % 27], sred[i]);
+  if (threadIdx.x < kC) atomicAdd(&db1[threadIdx.x], sred[kC * 3 * 9 + threadIdx.x]);
 }
 
 __global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
@@ -1175,13 +1429,12 @@ __global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, 
   }
 }
 
-int grid_for_elems(long long n) {
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const long long want = (n + 255) / 256;
-  const long long cap = 8LL * (sms > 0 ? sms : 152);
-  return static_cast<int>(want < cap ? (want > 0 ? want : 1) : cap);
+int sm_count();
+
+// CTAs of a tile kernel: at most per_sm resident ones per SM, each taking tiles in turn
+int tile_ctas(int batch, int w, int h, int tw, int th, int per_sm) {
+  const long long tiles = tile_grid(batch, w, h, tw, th).count, cap = static_cast<long long>(per_sm) * sm_count();
+  return static_cast<int>(tiles < cap ? tiles : cap);
 }
 
 int sm_count() {
@@ -1197,25 +1450,23 @@ int param_count() { return kParams; }
 
 size_t workspace_bytes(int batch, int width, int height) {
   const size_t n = static_cast<size_t>(batch) * width * height;
-  // X (float4), A1, A2, A3 (32 x BF16), r / dr (float), dA x 2 (32 x BF16)
-  return n * (16 + 3 * 64 + 4 + 2 * 64) + 4096;
+  // A1, A2, A3 (32 x BF16), dA x 2 (32 x BF16)
+  return n * (3 * 64 + 2 * 64) + 4096;
 }
 
-static void carve(unsigned char* ws, size_t n, float4** X, __nv_bfloat16** A1, __nv_bfloat16** A2,
-                  __nv_bfloat16** A3, float** r, __nv_bfloat16** G1, __nv_bfloat16** G2) {
+static void carve(unsigned char* ws, size_t n, __nv_bfloat16** A1, __nv_bfloat16** A2, __nv_bfloat16** A3,
+                  __nv_bfloat16** G1, __nv_bfloat16** G2) {
   size_t o = 0;
   auto take = [&](size_t bytes) {
     unsigned char* p = ws + o;
     o += (bytes + 255) & ~static_cast<size_t>(255);
-    return p;
+    return reinterpret_cast<__nv_bfloat16*>(p);
   };
-  *X = reinterpret_cast<float4*>(take(n * 16));
-  *A1 = reinterpret_cast<__nv_bfloat16*>(take(n * 64));
-  *A2 = reinterpret_cast<__nv_bfloat16*>(take(n * 64));
-  *A3 = reinterpret_cast<__nv_bfloat16*>(take(n * 64));
-  *r = reinterpret_cast<float*>(take(n * 4));
-  *G1 = reinterpret_cast<__nv_bfloat16*>(take(n * 64));
-  *G2 = reinterpret_cast<__nv_bfloat16*>(take(n * 64));
+  *A1 = take(n * 64);
+  *A2 = take(n * 64);
+  *A3 = take(n * 64);
+  *G1 = take(n * 64);
+  *G2 = take(n * 64);
 }
 
 cudaError_t pack_weights(const float* params, __nv_bfloat16* packed, cudaStream_t s) {
@@ -1231,20 +1482,21 @@ cudaError_t forward(const float* params, const __nv_bfloat16* packed, const floa
                     cudaStream_t s) {
   const size_t n = static_cast<size_t>(batch) * width * height;
   if (n > 0x7fffffffULL) return cudaErrorInvalidValue;  // the layers' pixel arithmetic is 32-bit
-  float4* X;
   __nv_bfloat16 *A1, *A2, *A3, *G1, *G2;
-  float* r;
-  carve(ws, n, &X, &A1, &A2, &A3, &r, &G1, &G2);
-  const int grid = grid_for_elems(static_cast<long long>(n));
-  pack_input_kernel<<<grid, 256, 0, s>>>(depth, X, batch, width, height);
-  conv_in_kernel<<<grid, 256, 0, s>>>(X, params, A1, batch, width, height);
+  carve(ws, n, &A1, &A2, &A3, &G1, &G2);
+  conv_in_kernel<<<tile_ctas(batch, width, height, kTileW, kTileH, 2), kTileThreads, 0, s>>>(depth, params, A1, batch, width,
+                                                                                          height);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = launch_conv32(A1, packed, params + kOffB2, nullptr, A2, batch, width, height, kForward, 1, error, s);
   if (e == cudaSuccess) {
     e = launch_conv32(A2, packed + 9 * kC * kC, params + kOffB3, nullptr, A3, batch, width, height, kForward, 1, error, s);
   }
   if (e != cudaSuccess) return e;
-  conv_out_kernel<<<grid, 256, 0, s>>>(A3, params, depth, fallback, out, batch, width, height);
+  static const cudaError_t attr =
+      cudaFuncSetAttribute(conv_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kOutSmem);
+  if (attr != cudaSuccess) return attr;
+  conv_out_kernel<<<tile_ctas(batch, width, height, kOutW, kOutH, kOutCtas), kTileThreads, kOutSmem, s>>>(
+      A3, params, depth, fallback, out, batch, width, height);
   return cudaGetLastError();
 }
 
@@ -1252,20 +1504,17 @@ cudaError_t backward(const float* params, const __nv_bfloat16* packed, const flo
                      const float* out, int batch, int width, int height, unsigned char* ws, float* grads, float* loss,
                      unsigned int* error, cudaStream_t s) {
   const size_t n = static_cast<size_t>(batch) * width * height;
-  float4* X;
   __nv_bfloat16 *A1, *A2, *A3, *G1, *G2;
-  float* dr;
-  carve(ws, n, &X, &A1, &A2, &A3, &dr, &G1, &G2);
-  const int grid = grid_for_elems(static_cast<long long>(n));
+  carve(ws, n, &A1, &A2, &A3, &G1, &G2);
   cudaError_t e = cudaMemsetAsync(grads, 0, kParams * sizeof(float), s);
   if (e == cudaSuccess) e = cudaMemsetAsync(loss, 0, 2 * sizeof(float), s);
   if (e != cudaSuccess) return e;
-  const int wg = 4 * sm_count();  // CUDA-core weight gradients: 256-thread CTAs, four per SM
-  loss_grad_kernel<<<grid, 256, 0, s>>>(out, target, depth, dr, static_cast<long long>(n), loss);
-  // layer 4: weights, then the gradient into A3
-  wgrad_kernel<kC, 1, true, false, 8><<<wg, kC * 8, 0, s>>>(A3, dr, grads + kOffW4, grads + kOffB4, batch, width,
-                                                             height);
-  dgrad_out_kernel<<<grid, 256, 0, s>>>(dr, params, A3, G1, batch, width, height);
+  // the loss, layer 4's weights and the gradient into A3
+  static const cudaError_t attr =
+      cudaFuncSetAttribute(out_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kOutBackSmem);
+  if (attr != cudaSuccess) return attr;
+  out_backward_kernel<<<tile_ctas(batch, width, height, kTileW, kTileH, 2), kTileThreads, kOutBackSmem, s>>>(
+      A3, params, depth, target, out, G1, grads + kOffW4, grads + kOffB4, loss, batch, width, height);
   // layer 3
   e = cudaGetLastError();
   if (e == cudaSuccess) e = launch_wgrad32(A2, G1, grads + kOffW3, grads + kOffB3, batch, width, height, error, s);
@@ -1280,8 +1529,8 @@ cudaError_t backward(const float* params, const __nv_bfloat16* packed, const flo
   }
   if (e != cudaSuccess) return e;
   // layer 1
-  wgrad_kernel<kCin, kC, false, true, 2><<<wg, kCin * kC * 2, 0, s>>>(X, G1, grads + kOffW1, grads + kOffB1, batch, width,
-                                                              height);
+  wgrad_in_kernel<<<tile_ctas(batch, width, height, kTileW, kWgInH, 2), kTileThreads, 0, s>>>(
+      depth, G1, grads + kOffW1, grads + kOffB1, batch, width, height);
   return cudaGetLastError();
 }
 
