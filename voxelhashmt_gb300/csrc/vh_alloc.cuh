@@ -35,8 +35,10 @@ __device__ __forceinline__ uint32_t smem_hash(unsigned long long k, int bits) {
 }
 
 // slot was found or inserted this frame: put it on the visible list once (the exchange both tests and sets the
-// slot's frame stamp: one round trip to L2)
-__device__ __forceinline__ void mark_visible(const Volume& V, uint32_t slot, uint32_t frame) {
+// slot's frame stamp: one round trip to L2).  stamp: the slot's stamp as loaded with its key; a block that several
+// tiles touch is mostly on the list already, which takes no atomic.
+__device__ __forceinline__ void mark_visible(const Volume& V, uint32_t slot, uint32_t frame, uint32_t stamp) {
+  if (stamp == frame) return;
   if (atomicExch(&V.slot_stamp[slot], frame) == frame) return;
   const uint32_t pos = atomicAdd(&V.counters->visible_count, 1U);
   V.visible[pos] = slot;
@@ -49,6 +51,7 @@ __device__ inline void insert_global(const Volume& V, unsigned long long key, ui
   uint32_t slot = hash_block_key(x, y, z) & V.mask;
   for (uint32_t probe = 0; probe < V.capacity; ++probe) {
     unsigned long long cur = *reinterpret_cast<volatile unsigned long long*>(&V.slot_keys[slot]);
+    const uint32_t stamp = *reinterpret_cast<volatile uint32_t*>(&V.slot_stamp[slot]);
     if (cur == kEmptyKey) {
       cur = atomicCAS(&V.slot_keys[slot], kEmptyKey, key);
       if (cur == kEmptyKey) {
@@ -64,12 +67,12 @@ __device__ inline void insert_global(const Volume& V, unsigned long long key, ui
           }
         }
         V.slot_block[slot] = idx;
-        mark_visible(V, slot, frame);
+        mark_visible(V, slot, frame, stamp);
         return;
       }
     }
     if (cur == key) {
-      mark_visible(V, slot, frame);
+      mark_visible(V, slot, frame, stamp);
       return;
     }
     slot = (slot + 1U) & V.mask;
@@ -77,12 +80,17 @@ __device__ inline void insert_global(const Volume& V, unsigned long long key, ui
   atomicOr(&V.counters->error, kErrHashFull);
 }
 
-// shared-memory set insert; returns 1 if inserted, 0 if present, -1 if the probe budget ran out
+// shared-memory set insert; returns 1 if inserted, 0 if present, -1 if the probe budget ran out.  A slot is read
+// before it is exchanged: most samples of a tile bring a key that is there already, and 32 lanes that exchange on one
+// address take turns where 32 reads of it are one (with the stamp check above: 110 -> 104 us a frame in the exact build
+// and 32 -> 31 in the fast-math one, 640x480 room).
 __device__ __forceinline__ int smem_insert(unsigned long long* set, int bits, unsigned long long key) {
   const uint32_t mask = (1U << bits) - 1U;
   uint32_t s = smem_hash(key, bits);
   for (int probe = 0; probe < kMaxSmemProbes; ++probe) {
-    const unsigned long long prev = atomicCAS(&set[s], kEmptyKey, key);
+    unsigned long long prev = *reinterpret_cast<volatile unsigned long long*>(&set[s]);
+    if (prev == key) return 0;
+    if (prev == kEmptyKey) prev = atomicCAS(&set[s], kEmptyKey, key);
     if (prev == kEmptyKey) return 1;
     if (prev == key) return 0;
     s = (s + 1U) & mask;
