@@ -178,3 +178,46 @@ def test_denoiser_layers_at_tile_edges(env, shape):
         a, r = got[off:off + n].astype(np.float64), ref[off:off + n]
         assert np.linalg.norm(a - r) <= 2e-2 * np.linalg.norm(r) + 1e-12, (off, n)
         off += n
+
+
+@pytest.mark.parametrize("form", ["plain", "chosen"])
+@pytest.mark.parametrize("size", [(5, 3), (64, 48)])
+def test_back_to_back_frames_equal_single_ones(env, small_orbit, form, size):
+    """Frames enqueued without a wait between them, of two volumes on two streams, the one depth buffer rewritten on the
+    stream between its frames and small enough that each kernel of a frame starts while the one before it runs: the same
+    blocks, word for word, as with a wait after every frame."""
+    backend, O = env
+    from voxelhashmt_gb300 import _capi, scenes
+    sc = small_orbit
+    w, h = size
+    K = scenes.Intrinsics(w, h, 55.4 * w / 64, 55.4 * w / 64, (w - 1) / 2.0, (h - 1) / 2.0)
+    on = int(form == "chosen")
+    algorithm = _capi.default_algorithm(allocation_mode=on, normal_mode=on, fast_math=on, autotune=0)
+    rng = np.random.default_rng(5)
+    depths = torch.from_numpy(np.stack([scenes.render_depth(sc, f)[:h, :w] for f in range(12)])).cuda()
+    depths = depths + torch.from_numpy(rng.normal(0, 1e-3, tuple(depths.shape)).astype(np.float32)).cuda()
+
+    def volume():
+        return backend.VoxelHashTSDF(sc.voxel_size, sc.truncation, hash_buckets=1 << 16, max_blocks=8192, layer_format=on,
+                                     algorithm=algorithm)
+
+    single = volume()
+    for f in range(12):
+        backend.integrate_depth_frame_cuda(single, backend.DepthFrame(K, depths[f].contiguous()), sc.poses[f])
+    want = O.sort_blocks(*single.export_blocks())
+    torch.cuda.synchronize()
+    vols, streams = [volume(), volume()], [torch.cuda.Stream(), torch.cuda.Stream()]
+    bufs = [torch.zeros((h, w), device="cuda") for _ in vols]
+    torch.cuda.synchronize()
+    for f in range(12):
+        for vol, st, buf in zip(vols, streams, bufs):
+            with torch.cuda.stream(st):
+                buf.copy_(depths[f])
+            backend.integrate_depth_frame_cuda(vol, backend.DepthFrame(K, buf), sc.poses[f], stream=st, synchronize=False)
+    for vol, st in zip(vols, streams):
+        vol.synchronize(st)
+        got = O.sort_blocks(*vol.export_blocks())
+        assert np.array_equal(got[0], want[0])
+        assert np.array_equal(got[1], want[1])
+        vol.close()
+    single.close()

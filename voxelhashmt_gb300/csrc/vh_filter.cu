@@ -23,6 +23,8 @@ __global__ void __launch_bounds__(kTX* kTY) filter_kernel(const float* __restric
                                                           const Params p, Counters* counters) {
   __shared__ filt::Smem S;
   const int tid = threadIdx.y * kTX + threadIdx.x;
+  allow_next();
+  wait_previous();
   if (kBeginFrame && blockIdx.x == 0 && blockIdx.y == 0 && tid == 0) filt::begin_frame(counters);
   filt::filter_tile(in, out, p, blockIdx.x * kTX, blockIdx.y * kTY, tid, S);
 }
@@ -44,7 +46,10 @@ __global__ void __launch_bounds__(kTX* kTY) normals_kernel(const float* __restri
   valid[ci] = n.w != 0.0f ? 1 : 0;
 }
 
-__global__ void begin_frame_kernel(Counters* counters) { filt::begin_frame(counters); }
+__global__ void begin_frame_kernel(Counters* counters) {
+  allow_next();
+  filt::begin_frame(counters);
+}
 
 }  // namespace
 
@@ -52,12 +57,8 @@ cudaError_t launch_filter(const float* in, float* out, const Params& p, Counters
   if (p.filter_radius < 0 || p.filter_radius > kR) return cudaErrorInvalidValue;
   const dim3 block(kTX, kTY);
   const dim3 grid((p.width + kTX - 1) / kTX, (p.height + kTY - 1) / kTY);
-  if (begin_frame) {
-    filter_kernel<true><<<grid, block, 0, s>>>(in, out, p, begin_frame);
-  } else {
-    filter_kernel<false><<<grid, block, 0, s>>>(in, out, p, nullptr);
-  }
-  return cudaGetLastError();
+  return launch_dependent(begin_frame ? filter_kernel<true> : filter_kernel<false>, grid, block, s, in, out, p,
+                          begin_frame);
 }
 
 cudaError_t launch_depth_normals(const float* in, float* normals, unsigned char* valid, const Params& p,

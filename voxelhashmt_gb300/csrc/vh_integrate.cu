@@ -687,6 +687,8 @@ __device__ __forceinline__ int voxel_observation(const float* __restrict__ depth
 // columns 32, 64, 128, 256 and as many rows a fifth of the warps of a 320x240 frame had one.
 __global__ void __launch_bounds__(kThreads) classify_kernel(const float* __restrict__ depth, const Volume V,
                                                             const Params p) {
+  allow_next();
+  wait_previous();
   const uint32_t nvis = V.counters->visible_count;
   const unsigned long long total = static_cast<unsigned long long>(nvis) * kBlockVoxels;
   const int lane = threadIdx.x & 31;
@@ -741,13 +743,14 @@ template <bool kFp16>
 __global__ void __launch_bounds__(kUpdateThreads, kUpdateMinB) update_kernel(const float* __restrict__ depth, const Volume V,
                                                                    const Params p) {
   __shared__ NormalScratch<kUpdateThreads> S;
+  const float gs[3] = {gaussian(0.0f, p.normal_k_spatial), gaussian(1.0f, p.normal_k_spatial),
+                       gaussian(2.0f, p.normal_k_spatial)};
+  const CameraDiv cam = camera_div(p);
+  wait_previous();
   const uint32_t n = V.counters->active_voxels, n_literal = V.counters->literal_voxels;
   const uint32_t literal_chunks = (n_literal + 31U) / 32U, chunks = literal_chunks + (n + 31U) / 32U;
   const uint32_t last = V.max_blocks * static_cast<uint32_t>(kBlockVoxels) - 1U;
   const int lane = threadIdx.x & 31;
-  const float gs[3] = {gaussian(0.0f, p.normal_k_spatial), gaussian(1.0f, p.normal_k_spatial),
-                       gaussian(2.0f, p.normal_k_spatial)};
-  const CameraDiv cam = camera_div(p);
   uint32_t sum_updated = 0U, sum_newly = 0U;
   uint32_t next = 0U;
   if (lane == 0) next = atomicAdd(&V.counters->update_queue, 1U);
@@ -902,6 +905,8 @@ __device__ __forceinline__ void map_tile(const float* __restrict__ depth, const 
 __global__ void __launch_bounds__(kMapTX * kMapTY) pixel_normal_kernel(const float* __restrict__ depth, const Params p,
                                                                        float4* __restrict__ nmap) {
   __shared__ MapSmem S;
+  allow_next();
+  wait_previous();
   map_tile(depth, p, nmap, blockIdx.x * kMapTX, blockIdx.y * kMapTY, threadIdx.y * kMapTX + threadIdx.x, S);
 }
 
@@ -912,6 +917,8 @@ __global__ void __launch_bounds__(kMapTX * kMapTY) map_prepare_kernel(const floa
                                                                       const Params p, float4* __restrict__ nmap) {
   __shared__ MapSmem S;
   const int tid = threadIdx.y * kMapTX + threadIdx.x;
+  allow_next();
+  wait_previous();
   const uint32_t nvis = V.counters->visible_count;
   const uint32_t nthreads = gridDim.x * gridDim.y * kMapTX * kMapTY;
   for (uint32_t i = (blockIdx.y * gridDim.x + blockIdx.x) * (kMapTX * kMapTY) + tid; i < nvis; i += nthreads) {
@@ -1041,6 +1048,7 @@ __global__ void __launch_bounds__(kT, kMinBlocks) fused_update_kernel(const floa
   __shared__ MapQueue<kT, kS> Q;
   __shared__ uint32_t s_item;
   __shared__ CtaStats s_stats;
+  wait_previous();
   const uint32_t nvis = V.counters->visible_count;
   const uint32_t nchunks = nvis * static_cast<uint32_t>(kBlockVoxels / kChunk);
   const int tid = threadIdx.x, lane = tid & 31;
@@ -1167,6 +1175,7 @@ __device__ __forceinline__ void copy_desc(SceneDesc& dst, const SceneDesc* __res
 // allocation of the step touches a scene's counters)
 __global__ void batch_begin_kernel(const SceneDesc* __restrict__ descs, const BatchHeader* __restrict__ hdr,
                                    uint32_t* __restrict__ queue) {
+  allow_next();
   if (threadIdx.x < 3) queue[threadIdx.x] = 0U;
   const int nsc = static_cast<int>(hdr->nscenes);
   for (int k = threadIdx.x; k < nsc; k += blockDim.x) {
@@ -1229,6 +1238,8 @@ __global__ void __launch_bounds__(filt::kTX * filt::kTY) batch_filter_alloc_kern
   __shared__ SceneDesc D;
   __shared__ uint32_t s_item;
   __shared__ int s_scene;
+  allow_next();
+  wait_previous();
   batch_filter_alloc_body<kBand>(descs, hdr, queue, S, D, s_item, s_scene);
 }
 
@@ -1282,6 +1293,8 @@ __global__ void __launch_bounds__(kMapTX * kMapTY) batch_map_kernel(const SceneD
   __shared__ SceneDesc D;
   __shared__ uint32_t s_item;
   __shared__ int s_scene;
+  allow_next();
+  wait_previous();
   batch_map_body(descs, hdr, queue, M, D, s_item, s_scene);
 }
 
@@ -1416,6 +1429,7 @@ __global__ void __launch_bounds__(kUT, kUMinB) batch_update_kernel(const SceneDe
   __shared__ SceneDesc D;
   __shared__ uint32_t s_item;
   __shared__ int s_scene;
+  wait_previous();
   batch_update_body<kUT>(descs, hdr, queue, U, D, s_item, s_scene);
 }
 
@@ -1531,8 +1545,10 @@ __global__ void __launch_bounds__(filt::kTX * filt::kTY) filter_alloc_kernel(con
   } S;
   const int tid = threadIdx.x;
   const int u0 = blockIdx.x * filt::kTX, v0 = blockIdx.y * filt::kTY;
+  allow_next();
   const float d = filt::filter_tile(in, out, p, u0, v0, tid, S.f);
   __syncthreads();  // the filter's staged tiles become the allocation's sets
+  wait_previous();  // the frame has begun: the filter does not depend on it
   const int u = u0 + tid % filt::kTX, v = v0 + tid / filt::kTX;
   const bool has = u < p.width && v < p.height && u % p.stride == 0 && v % p.stride == 0 &&
                    u / p.stride < p.sample_width && v / p.stride < p.sample_height;
@@ -1567,18 +1583,13 @@ cudaError_t launch_filter_alloc(const float* in, float* out, const Volume& V, co
   const cudaError_t e = launch_begin_frame(V.counters, s);
   if (e != cudaSuccess) return e;
   const dim3 grid((p.width + filt::kTX - 1) / filt::kTX, (p.height + filt::kTY - 1) / filt::kTY);
-  if (p.alloc_mode == 1) {
-    filter_alloc_kernel<true><<<grid, filt::kTX * filt::kTY, 0, s>>>(in, out, V, p);
-  } else {
-    filter_alloc_kernel<false><<<grid, filt::kTX * filt::kTY, 0, s>>>(in, out, V, p);
-  }
-  return cudaGetLastError();
+  return launch_dependent(p.alloc_mode == 1 ? filter_alloc_kernel<true> : filter_alloc_kernel<false>, grid,
+                          dim3(filt::kTX * filt::kTY), s, in, out, V, p);
 }
 
 cudaError_t launch_pixel_normals(const float* depth, const Params& p, float4* nmap, cudaStream_t s) {
   const dim3 mb(kMapTX, kMapTY), mg((p.width + kMapTX - 1) / kMapTX, (p.height + kMapTY - 1) / kMapTY);
-  pixel_normal_kernel<<<mg, mb, 0, s>>>(depth, p, nmap);
-  return cudaGetLastError();
+  return launch_dependent(pixel_normal_kernel, mg, mb, s, depth, p, nmap);
 }
 
 // first kernel of the update: the active-voxel list (classify_kernel) or the per-pixel normal map with the
@@ -1588,13 +1599,11 @@ cudaError_t launch_integrate_prepare(const float* depth, const Volume& V, const 
   if (p.normal_mode == 1) {
     if (nmap == nullptr) return cudaErrorInvalidValue;
     const dim3 mb(kMapTX, kMapTY), mg((p.width + kMapTX - 1) / kMapTX, (p.height + kMapTY - 1) / kMapTY);
-    map_prepare_kernel<<<mg, mb, 0, s>>>(depth, V, p, nmap);
-    return cudaGetLastError();
+    return launch_dependent(map_prepare_kernel, mg, mb, s, depth, V, p, nmap);
   }
   static int classify_grid = 0;
   if (classify_grid == 0) classify_grid = grid_for(reinterpret_cast<const void*>(classify_kernel), kThreads);
-  classify_kernel<<<classify_grid, kThreads, 0, s>>>(depth, V, p);
-  return cudaGetLastError();
+  return launch_dependent(classify_kernel, dim3(classify_grid), dim3(kThreads), s, depth, V, p);
 }
 
 // second kernel: the layer update over the active list (update_kernel) or over every visible voxel with the
@@ -1603,14 +1612,15 @@ cudaError_t launch_integrate_prepare(const float* depth, const Volume& V, const 
 // SM).  The grid is always the number of CTAs that fit on the device at once.
 struct FusedVariant {
   const void* fn;
-  void (*launch)(int grid, cudaStream_t s, const float* depth, const float4* nmap, const Volume& V, const Params& p);
+  cudaError_t (*launch)(int grid, cudaStream_t s, const float* depth, const float4* nmap, const Volume& V,
+                        const Params& p);
   int threads;
 };
 
 template <int kT, int kMinB, int kS>
-void launch_fused_variant(int grid, cudaStream_t s, const float* depth, const float4* nmap, const Volume& V,
-                          const Params& p) {
-  fused_update_kernel<kT, kMinB, kS><<<grid, kT, 0, s>>>(depth, nmap, V, p);
+cudaError_t launch_fused_variant(int grid, cudaStream_t s, const float* depth, const float4* nmap, const Volume& V,
+                                 const Params& p) {
+  return launch_dependent(fused_update_kernel<kT, kMinB, kS>, dim3(grid), dim3(kT), s, depth, nmap, V, p);
 }
 
 // (threads per CTA, minimum resident CTAs per SM, voxel slots per thread and pass)
@@ -1643,16 +1653,11 @@ cudaError_t launch_integrate_update(const float* depth, const Volume& V, const P
     static int fused_grid[kNumFusedVariants] = {};
     const FusedVariant& fv = kFusedVariants[variant];
     if (fused_grid[variant] == 0) fused_grid[variant] = grid_for(fv.fn, fv.threads);
-    fv.launch(grid > 0 ? grid : fused_grid[variant], s, depth, nmap, V, p);
-    return cudaGetLastError();
+    return fv.launch(grid > 0 ? grid : fused_grid[variant], s, depth, nmap, V, p);
   }
   const int g = grid > 0 ? grid : integrate_grid_size();
-  if (V.layers16 != nullptr) {
-    update_kernel<true><<<g, kUpdateThreads, 0, s>>>(depth, V, p);
-  } else {
-    update_kernel<false><<<g, kUpdateThreads, 0, s>>>(depth, V, p);
-  }
-  return cudaGetLastError();
+  return launch_dependent(V.layers16 != nullptr ? update_kernel<true> : update_kernel<false>, dim3(g), dim3(kUpdateThreads),
+                          s, depth, V, p);
 }
 
 // launch shape of batch_update_kernel: threads per CTA (the chunk of voxel slots) and resident CTAs per SM
@@ -1667,14 +1672,14 @@ cudaError_t launch_batch(const SceneDesc* descs, const BatchHeader* hdr, uint32_
     grids[3] = grid_for(reinterpret_cast<const void*>(batch_update_kernel<kBatchUT, kBatchUMinB>), kBatchUT);
   }
   batch_begin_kernel<<<1, 256, 0, s>>>(descs, hdr, queue);
-  if (band) {
-    batch_filter_alloc_kernel<true><<<grids[1], filt::kTX * filt::kTY, 0, s>>>(descs, hdr, queue);
-  } else {
-    batch_filter_alloc_kernel<false><<<grids[0], filt::kTX * filt::kTY, 0, s>>>(descs, hdr, queue);
-  }
-  batch_map_kernel<<<grids[2], kMapTX * kMapTY, 0, s>>>(descs, hdr, queue);
-  batch_update_kernel<kBatchUT, kBatchUMinB><<<grids[3], kBatchUT, 0, s>>>(descs, hdr, queue);
-  return cudaGetLastError();
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  e = launch_dependent(band ? batch_filter_alloc_kernel<true> : batch_filter_alloc_kernel<false>, grids[band ? 1 : 0],
+                       filt::kTX * filt::kTY, s, descs, hdr, queue);
+  if (e != cudaSuccess) return e;
+  e = launch_dependent(batch_map_kernel, grids[2], kMapTX * kMapTY, s, descs, hdr, queue);
+  if (e != cudaSuccess) return e;
+  return launch_dependent(batch_update_kernel<kBatchUT, kBatchUMinB>, grids[3], kBatchUT, s, descs, hdr, queue);
 }
 
 // The step as one cooperative launch of batch_persistent_kernel (queue: 3 work-queue words; bar: 2 barrier words,
