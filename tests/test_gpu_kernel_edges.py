@@ -221,3 +221,39 @@ def test_back_to_back_frames_equal_single_ones(env, small_orbit, form, size):
         assert np.array_equal(got[1], want[1])
         vol.close()
     single.close()
+
+
+@pytest.mark.parametrize("radius", [0, 1, 2])
+@pytest.mark.parametrize("size", [(1, 1), (3, 2), (8, 4), (9, 5), (31, 17), (729, 312), (737, 312)])
+def test_filter_and_normals_of_small_and_large_tiles(env, radius, size):
+    """The depth filter and the pixel normals with tiles of 8x4 pixels (up to 912 tiles of 32x8, as at 729x312: 23 by 39
+    = 897) and of 32x8 (737x312: 24 by 39 = 936), with holes, steps, infinities, NaN and negative depth: word for word
+    the oracle's."""
+    backend, O = env
+    from voxelhashmt_gb300 import _capi, scenes
+    w, h = size
+    rng = np.random.default_rng(w * 7 + h)
+    depth = (1.0 + 0.2 * np.sin(np.arange(w) / 7.0)[None, :] + 0.01 * rng.normal(size=(h, w))).astype(np.float32)
+    depth[rng.random((h, w)) < 0.05] = 0.0
+    depth[rng.random((h, w)) < 0.05] += 0.3
+    if w > 30:
+        depth[5, 7], depth[6, 20], depth[9, 9] = np.inf, np.nan, -1.0
+    K = scenes.Intrinsics(w, h, 500.0, 490.0, 20.0, 10.0)
+    vol = backend.VoxelHashTSDF(0.01, 0.03, hash_buckets=1 << 10, max_blocks=64,
+                                algorithm=_capi.default_algorithm(filter_radius=radius))
+    finite = np.where(np.isinf(depth), np.float32(0.0), depth)  # a map's taps are pixels, the oracle's are blends of two
+    src, fin = torch.from_numpy(depth).cuda(), torch.from_numpy(finite).cuda()
+    out, nrm = torch.full_like(src, -7.0), torch.full((h, w, 4), -7.0, device="cuda")
+    torch.cuda.synchronize()
+    Ki = _capi.intrinsics(K)
+    for fn, a, dst in ((_capi.lib().vh_filter_depth, src, out), (_capi.lib().vh_pixel_normals, fin, nrm)):
+        _capi.check(fn(vol.handle, C.c_void_p(a.data_ptr()), C.c_void_p(dst.data_ptr()), C.byref(Ki), None), vol.handle)
+    vol.synchronize()
+    vol.close()
+    cfg = O.config(O.FLAVOR_REF_GPU, O.EXP_OWN, threads=8, filter_radius=radius)
+    assert np.array_equal(out.cpu().numpy(), O.filter_depth(cfg, depth, K), equal_nan=True)
+    if radius == 2:
+        want, ok = O.pixel_normals(cfg, finite, K)
+        got = nrm.cpu().numpy()
+        assert np.array_equal(got[..., 3], ok.astype(np.float32))
+        assert np.array_equal(_bits(got[..., :3][ok != 0]), _bits(want[ok != 0]))

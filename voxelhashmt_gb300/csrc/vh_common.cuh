@@ -620,4 +620,11 @@ inline cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 b
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
 }
 
+// An image of so few 32x8 tiles that the tiles of 8x4 pixels with a warp per tap (filter_small_tile, map_tile_small) are
+// the faster ones: six large tiles per SM, of the eight that are resident at once.  The bilateral filter and the
+// normal map of the exact build took, with large and with small tiles (us): 160x120 (75 tiles) 32 and 15, 320x240 (300)
+// 68 and 33, 480x360 (675) 73 and 65, 640x480 (1,200) 103 and 109, 1280x960 347 and 404 (the small tiles' halo is
+// three times their area, the large ones' 1.7).  The normal map of the fast-math build crosses at the same size.
+inline bool few_tiles(dim3 large) { return static_cast<unsigned long long>(large.x) * large.y <= 6ULL * 152ULL; }
+
 }  // namespace vh

@@ -29,6 +29,17 @@ __global__ void __launch_bounds__(kTX* kTY) filter_kernel(const float* __restric
   filt::filter_tile(in, out, p, blockIdx.x * kTX, blockIdx.y * kTY, tid, S);
 }
 
+template <bool kBeginFrame>
+__global__ void __launch_bounds__(filt::kSmallThreads) filter_small_kernel(const float* __restrict__ in,
+                                                                           float* __restrict__ out, const Params p,
+                                                                           Counters* counters) {
+  __shared__ filt::SmallSmem S;
+  allow_next();
+  wait_previous();
+  if (kBeginFrame && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) filt::begin_frame(counters);
+  filt::filter_small_tile(in, out, p, blockIdx.x * filt::kSmallTX, blockIdx.y * filt::kSmallTY, threadIdx.x, S);
+}
+
 __global__ void __launch_bounds__(kTX* kTY) normals_kernel(const float* __restrict__ in, float* __restrict__ normals,
                                                            unsigned char* __restrict__ valid, const Params p) {
   __shared__ float s_depth[kDH][kDW];
@@ -57,6 +68,11 @@ cudaError_t launch_filter(const float* in, float* out, const Params& p, Counters
   if (p.filter_radius < 0 || p.filter_radius > kR) return cudaErrorInvalidValue;
   const dim3 block(kTX, kTY);
   const dim3 grid((p.width + kTX - 1) / kTX, (p.height + kTY - 1) / kTY);
+  if (few_tiles(grid)) {
+    const dim3 small((p.width + filt::kSmallTX - 1) / filt::kSmallTX, (p.height + filt::kSmallTY - 1) / filt::kSmallTY);
+    return launch_dependent(begin_frame ? filter_small_kernel<true> : filter_small_kernel<false>, small,
+                            filt::kSmallThreads, s, in, out, p, begin_frame);
+  }
   return launch_dependent(begin_frame ? filter_kernel<true> : filter_kernel<false>, grid, block, s, in, out, p,
                           begin_frame);
 }

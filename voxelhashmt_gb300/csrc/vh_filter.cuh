@@ -23,7 +23,8 @@ constexpr int kNH = kTY + 2 * kR;
 
 // estimateSurfaceNormalAtPixel (cuda_tsdf_integrator.cu:581-627) on the staged tile; (sx, sy) = tile coords
 // of pixel (u, v) in s_depth.
-__device__ __forceinline__ float4 pixel_normal(const float (*s_depth)[kDW], int sx, int sy, int u, int v,
+template <int kPitch>
+__device__ __forceinline__ float4 pixel_normal(const float (*s_depth)[kPitch], int sx, int sy, int u, int v,
                                                const Params& p) {
   const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   if (u <= 0 || v <= 0 || u + 1 >= p.width || v + 1 >= p.height) return none;
@@ -112,6 +113,81 @@ __device__ __forceinline__ void bilateral_taps(const Smem& S, int tx, int ty, fl
     }
   }
 }
+
+#ifndef VH_FAST_MATH
+// The filter of a small image: a tile of 8x4 pixels, and each of its up to 25 taps' weights computed by a warp of its
+// own lanes (lane = pixel) into shared memory; one warp then adds them in the reference's order.  With 32x8 tiles and
+// a thread per pixel an image of 160x120 is 75 CTAs of 25 taps with two exponentials each, one after another: the time
+// of one long chain on half of the SMs (filter and normal map 32 us; 15 us with small tiles).
+constexpr int kSmallTX = 8, kSmallTY = 4, kSmallThreads = 288;
+
+struct SmallSmem {
+  float depth[kSmallTY + 2 * (kR + 1)][kSmallTX + 2 * (kR + 1)];
+  float4 normal[kSmallTY + 2 * kR][kSmallTX + 2 * kR];
+  float spatial[(2 * kR + 1) * (2 * kR + 1)];
+  float2 tap[(2 * kR + 1) * (2 * kR + 1)][kSmallTX * kSmallTY];  // weight * depth, weight
+};
+
+__device__ __forceinline__ void filter_small_tile(const float* __restrict__ in, float* __restrict__ out,
+                                                  const Params& p, int u0, int v0, int tid, SmallSmem& S) {
+  constexpr int kW = kSmallTX + 2 * (kR + 1), kH = kSmallTY + 2 * (kR + 1);
+  constexpr int kNx = kSmallTX + 2 * kR, kNy = kSmallTY + 2 * kR;
+  static_assert(kW * kH <= kSmallThreads && kSmallTX * kSmallTY == 32, "one pass to stage a tile, a lane per pixel");
+  if (tid < kW * kH) {
+    const int dy = tid / kW, dx = tid - dy * kW;
+    const int gu = u0 + dx - (kR + 1), gv = v0 + dy - (kR + 1);
+    S.depth[dy][dx] = (gu >= 0 && gu < p.width && gv >= 0 && gv < p.height)
+                          ? __ldg(&in[static_cast<size_t>(gv) * p.width + gu])
+                          : 0.0f;
+  } else if (tid < kW * kH + (2 * kR + 1) * (2 * kR + 1)) {
+    const int k = tid - kW * kH;
+    const int du = k % (2 * kR + 1) - kR, dv = k / (2 * kR + 1) - kR;
+    S.spatial[k] = gaussian(static_cast<float>(du * du + dv * dv), p.filter_k_spatial);
+  }
+  __syncthreads();
+  if (tid < kNx * kNy) {
+    const int ny = tid / kNx, nx = tid - ny * kNx;
+    S.normal[ny][nx] = pixel_normal(S.depth, nx + 1, ny + 1, u0 + nx - kR, v0 + ny - kR, p);
+  }
+  __syncthreads();
+  const int lane = tid & 31, tx = lane % kSmallTX, ty = lane / kSmallTX;
+  const float center = S.depth[ty + kR + 1][tx + kR + 1];
+  const float4 cn4 = S.normal[ty + kR][tx + kR];
+  const bool has_cn = cn4.w != 0.0f;
+  const float thr = disc_threshold(p, center);
+  const int side = 2 * p.filter_radius + 1, taps = side * side;
+#pragma unroll 1
+  for (int k = tid >> 5; k < taps; k += kSmallThreads / 32) {
+    const int dv = k / side - p.filter_radius, du = k % side - p.filter_radius;
+    const float sd = S.depth[ty + kR + 1 + dv][tx + kR + 1 + du];
+    float w = 0.0f, wd = 0.0f;
+    const float delta = sd - center;
+    const float range = delta * delta;
+    if (center > 0.0f && !(sd <= 0.0f) && !(fabsf(delta) > thr) && !gaussian_is_zero(range, p.filter_k_range)) {
+      const float4 sn = S.normal[ty + kR + dv][tx + kR + du];
+      const float cosine = clampf(dot3(mk3(cn4.x, cn4.y, cn4.z), mk3(sn.x, sn.y, sn.z)), -1.0f, 1.0f);
+      if (!has_cn || (sn.w != 0.0f && !(cosine < p.filter_min_cos))) {
+        w = S.spatial[(dv + kR) * (2 * kR + 1) + (du + kR)] * gaussian(range, p.filter_k_range);
+        const float ad = 1.0f - cosine;
+        if (has_cn) w *= gaussian(ad * ad, p.filter_k_angular);
+        wd = w * sd;
+      }
+    }
+    S.tap[k][lane] = make_float2(wd, w);
+  }
+  __syncthreads();
+  const int u = u0 + tx, v = v0 + ty;
+  if (tid >= 32 || u >= p.width || v >= p.height) return;
+  float wds = 0.0f, ws = 0.0f;  // a tap left out adds zeros
+#pragma unroll 5
+  for (int k = 0; k < taps; ++k) {
+    const float2 t = S.tap[k][lane];
+    wds += t.x;
+    ws += t.y;
+  }
+  out[static_cast<size_t>(v) * p.width + u] = center <= 0.0f ? 0.0f : (ws > 1e-6f ? wds / ws : center);
+}
+#endif
 
 // bilateralFilterDepthKernel (cuda_tsdf_integrator.cu:650-725) for the output tile at (u0, v0); every thread of
 // the CTA calls it (it synchronises); thread (tx, ty) = tid % kTX, tid / kTX writes pixel (u0 + tx, v0 + ty)

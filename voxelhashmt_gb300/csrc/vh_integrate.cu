@@ -828,46 +828,78 @@ struct MapSmem {
   unsigned char pv[kMapH][kMapW], nv[kMapH][kMapW];
 };
 
+// 1. the backprojected point of pixel (x, y), position (tx, ty) of the tile (invalid outside the image or where
+// depth <= 0)
+template <class Smem>
+__device__ __forceinline__ void map_point(const float* __restrict__ depth, const Params& p, int x, int y, int tx, int ty,
+                                          Smem& S) {
+  float d = 0.0f;
+  if (x >= 0 && x < p.width && y >= 0 && y < p.height) d = __ldg(&depth[static_cast<size_t>(y) * p.width + x]);
+  const bool ok = d > 0.0f;
+  const f3 q = ok ? backproject(static_cast<float>(x), static_cast<float>(y), d, p) : mk3(0.0f, 0.0f, 0.0f);
+  S.px[ty][tx] = q.x;
+  S.py[ty][tx] = q.y;
+  S.pz[ty][tx] = q.z;
+  S.pv[ty][tx] = ok ? 1 : 0;
+}
+
+// 2. the base normal (estimateSurfaceNormalBaseCamera), oriented toward the camera; none on the tile's outer ring
+template <int kW, int kH, class Smem>
+__device__ __forceinline__ void map_base_normal(int tx, int ty, Smem& S) {
+  bool ok = tx >= 1 && tx < kW - 1 && ty >= 1 && ty < kH - 1 && S.pv[ty][tx] && S.pv[ty][tx - 1] && S.pv[ty][tx + 1] &&
+            S.pv[ty - 1][tx] && S.pv[ty + 1][tx];
+  f3 n = mk3(0.0f, 0.0f, 0.0f);
+  if (ok) {
+    const f3 dv = mk3(S.px[ty + 1][tx] - S.px[ty - 1][tx], S.py[ty + 1][tx] - S.py[ty - 1][tx],
+                      S.pz[ty + 1][tx] - S.pz[ty - 1][tx]);
+    const f3 du = mk3(S.px[ty][tx + 1] - S.px[ty][tx - 1], S.py[ty][tx + 1] - S.py[ty][tx - 1],
+                      S.pz[ty][tx + 1] - S.pz[ty][tx - 1]);
+    n = normalize3(cross3(dv, du));
+    ok = norm3(n) > 1e-6f;
+    if (ok) n = orient_unit_toward_camera(n, mk3(S.px[ty][tx], S.py[ty][tx], S.pz[ty][tx]));
+  }
+  S.nx[ty][tx] = n.x;
+  S.ny[ty][tx] = n.y;
+  S.nz[ty][tx] = n.z;
+  S.nv[ty][tx] = ok ? 1 : 0;
+}
+
+// 3. the bilateral combination of the 3x3 base normals (estimateSurfaceNormalCamera): the weight of neighbour k of
+// (cx, cy), and the normal from the weighted sum
+template <class Smem>
+__device__ __forceinline__ float map_tap_weight(const Params& p, const Smem& S, int cx, int cy, int k) {
+  const int dx = k % 3 - 1, dy = k / 3 - 1, sx = cx + dx, sy = cy + dy;
+  const float delta = S.pz[sy][sx] - S.pz[cy][cx];
+  const f3 cn = mk3(S.nx[cy][cx], S.ny[cy][cx], S.nz[cy][cx]), sn = mk3(S.nx[sy][sx], S.ny[sy][sx], S.nz[sy][sx]);
+  const float ad = 1.0f - clampf(dot3(cn, sn), -1.0f, 1.0f);
+  const int r2 = dx * dx + dy * dy;
+  return (r2 == 0 ? 1.0f : gaussian(static_cast<float>(r2), p.normal_k_spatial)) *
+         gaussian(delta * delta, p.normal_k_range) * gaussian(ad * ad, p.normal_k_angular);
+}
+
+__device__ __forceinline__ f3 map_combine(f3 cn, f3 cp, f3 wsum, float ws) {
+  f3 n = cn;
+  if (ws > 1e-6f) {
+    n = orient_toward_camera(normalize3(mul3(wsum, 1.0f / ws)), cp);
+    if (norm3(n) <= 1e-6f) n = cn;
+  }
+  return n;
+}
+
 // the normal map of the 32x8 pixel tile at (x0, y0); every thread of the CTA calls it (it synchronises)
 __device__ __forceinline__ void map_tile(const float* __restrict__ depth, const Params& p, float4* __restrict__ nmap,
                                          int x0t, int y0t, int tid, MapSmem& S) {
   const int x0 = x0t - kMapHalo, y0 = y0t - kMapHalo;
-  // 1. backprojected points of the tile + halo (invalid outside the image or where depth <= 0)
   for (int k = tid; k < kMapW * kMapH; k += kMapTX * kMapTY) {
     const int ty = k / kMapW, tx = k - ty * kMapW;
-    const int x = x0 + tx, y = y0 + ty;
-    float d = 0.0f;
-    if (x >= 0 && x < p.width && y >= 0 && y < p.height) d = __ldg(&depth[static_cast<size_t>(y) * p.width + x]);
-    const bool ok = d > 0.0f;
-    const f3 q = ok ? backproject(static_cast<float>(x), static_cast<float>(y), d, p) : mk3(0.0f, 0.0f, 0.0f);
-    S.px[ty][tx] = q.x;
-    S.py[ty][tx] = q.y;
-    S.pz[ty][tx] = q.z;
-    S.pv[ty][tx] = ok ? 1 : 0;
+    map_point(depth, p, x0 + tx, y0 + ty, tx, ty, S);
   }
   __syncthreads();
-  // 2. base normals (estimateSurfaceNormalBaseCamera) of the tile + 1-pixel ring, oriented toward the camera
   for (int k = tid; k < kMapW * kMapH; k += kMapTX * kMapTY) {
     const int ty = k / kMapW, tx = k - ty * kMapW;
-    bool ok = tx >= 1 && tx < kMapW - 1 && ty >= 1 && ty < kMapH - 1 && S.pv[ty][tx] && S.pv[ty][tx - 1] &&
-              S.pv[ty][tx + 1] && S.pv[ty - 1][tx] && S.pv[ty + 1][tx];
-    f3 n = mk3(0.0f, 0.0f, 0.0f);
-    if (ok) {
-      const f3 dv = mk3(S.px[ty + 1][tx] - S.px[ty - 1][tx], S.py[ty + 1][tx] - S.py[ty - 1][tx],
-                        S.pz[ty + 1][tx] - S.pz[ty - 1][tx]);
-      const f3 du = mk3(S.px[ty][tx + 1] - S.px[ty][tx - 1], S.py[ty][tx + 1] - S.py[ty][tx - 1],
-                        S.pz[ty][tx + 1] - S.pz[ty][tx - 1]);
-      n = normalize3(cross3(dv, du));
-      ok = norm3(n) > 1e-6f;
-      if (ok) n = orient_unit_toward_camera(n, mk3(S.px[ty][tx], S.py[ty][tx], S.pz[ty][tx]));
-    }
-    S.nx[ty][tx] = n.x;
-    S.ny[ty][tx] = n.y;
-    S.nz[ty][tx] = n.z;
-    S.nv[ty][tx] = ok ? 1 : 0;
+    map_base_normal<kMapW, kMapH>(tx, ty, S);
   }
   __syncthreads();
-  // 3. the bilateral combination of the 3x3 base normals (estimateSurfaceNormalCamera)
   const int lx = tid % kMapTX, ly = tid / kMapTX;
   const int x = x0t + lx, y = y0t + ly;
   if (x >= p.width || y >= p.height) return;
@@ -892,14 +924,65 @@ __device__ __forceinline__ void map_tile(const float* __restrict__ depth, const 
       wsum = add3(wsum, mul3(sn, w));
       ws += w;
     }
-    f3 n = cn;
-    if (ws > 1e-6f) {
-      n = orient_toward_camera(normalize3(mul3(wsum, 1.0f / ws)), cp);
-      if (norm3(n) <= 1e-6f) n = cn;
-    }
+    const f3 n = map_combine(cn, cp, wsum, ws);
     out = make_float4(n.x, n.y, n.z, 1.0f);
   }
   nmap[static_cast<size_t>(y) * p.width + x] = out;
+}
+
+// map_tile for a tile of 8x4 pixels: each of the 9 taps' weights by a warp of its own (lane = pixel), added in order by
+// one warp.
+constexpr int kSmallMapTX = 8, kSmallMapTY = 4, kSmallMapThreads = 288;
+constexpr int kSmallMapW = kSmallMapTX + 2 * kMapHalo, kSmallMapH = kSmallMapTY + 2 * kMapHalo;
+
+struct SmallMapSmem {
+  float px[kSmallMapH][kSmallMapW], py[kSmallMapH][kSmallMapW], pz[kSmallMapH][kSmallMapW];
+  float nx[kSmallMapH][kSmallMapW], ny[kSmallMapH][kSmallMapW], nz[kSmallMapH][kSmallMapW];
+  unsigned char pv[kSmallMapH][kSmallMapW], nv[kSmallMapH][kSmallMapW];
+  float w[9][kSmallMapTX * kSmallMapTY];
+};
+
+__device__ __forceinline__ void map_tile_small(const float* __restrict__ depth, const Params& p,
+                                               float4* __restrict__ nmap, int x0t, int y0t, int tid, SmallMapSmem& S) {
+  static_assert(kSmallMapTX * kSmallMapTY == 32 && kSmallMapThreads == 9 * 32, "a warp per tap, a lane per pixel");
+  const int ty = tid / kSmallMapW, tx = tid - ty * kSmallMapW;
+  if (ty < kSmallMapH) map_point(depth, p, x0t - kMapHalo + tx, y0t - kMapHalo + ty, tx, ty, S);
+  __syncthreads();
+  if (ty < kSmallMapH) map_base_normal<kSmallMapW, kSmallMapH>(tx, ty, S);
+  __syncthreads();
+  const int lane = tid & 31, k = tid >> 5;
+  const int lx = lane % kSmallMapTX, ly = lane / kSmallMapTX;
+  const int cx = lx + kMapHalo, cy = ly + kMapHalo;
+  S.w[k][lane] = map_tap_weight(p, S, cx, cy, k);
+  __syncthreads();
+  const int x = x0t + lx, y = y0t + ly;
+  if (tid >= 32 || x >= p.width || y >= p.height) return;
+  float4 out = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  if (S.nv[cy][cx]) {
+    f3 wsum = mk3(0.0f, 0.0f, 0.0f);
+    float ws = 0.0f;
+#pragma unroll
+    for (int t = 0; t < 9; ++t) {
+      const int sx = cx + t % 3 - 1, sy = cy + t / 3 - 1;
+      if (!S.nv[sy][sx]) continue;
+      const float w = S.w[t][lane];
+      wsum = add3(wsum, mul3(mk3(S.nx[sy][sx], S.ny[sy][sx], S.nz[sy][sx]), w));
+      ws += w;
+    }
+    const f3 n = map_combine(mk3(S.nx[cy][cx], S.ny[cy][cx], S.nz[cy][cx]), mk3(S.px[cy][cx], S.py[cy][cx], S.pz[cy][cx]),
+                             wsum, ws);
+    out = make_float4(n.x, n.y, n.z, 1.0f);
+  }
+  nmap[static_cast<size_t>(y) * p.width + x] = out;
+}
+
+__global__ void __launch_bounds__(kSmallMapThreads) pixel_normal_small_kernel(const float* __restrict__ depth,
+                                                                              const Params p,
+                                                                              float4* __restrict__ nmap) {
+  __shared__ SmallMapSmem S;
+  allow_next();
+  wait_previous();
+  map_tile_small(depth, p, nmap, blockIdx.x * kSmallMapTX, blockIdx.y * kSmallMapTY, threadIdx.x, S);
 }
 
 __global__ void __launch_bounds__(kMapTX * kMapTY) pixel_normal_kernel(const float* __restrict__ depth, const Params p,
@@ -1589,6 +1672,10 @@ cudaError_t launch_filter_alloc(const float* in, float* out, const Volume& V, co
 
 cudaError_t launch_pixel_normals(const float* depth, const Params& p, float4* nmap, cudaStream_t s) {
   const dim3 mb(kMapTX, kMapTY), mg((p.width + kMapTX - 1) / kMapTX, (p.height + kMapTY - 1) / kMapTY);
+  if (few_tiles(mg)) {
+    const dim3 small((p.width + kSmallMapTX - 1) / kSmallMapTX, (p.height + kSmallMapTY - 1) / kSmallMapTY);
+    return launch_dependent(pixel_normal_small_kernel, small, kSmallMapThreads, s, depth, p, nmap);
+  }
   return launch_dependent(pixel_normal_kernel, mg, mb, s, depth, p, nmap);
 }
 
