@@ -257,3 +257,32 @@ def test_filter_and_normals_of_small_and_large_tiles(env, radius, size):
         got = nrm.cpu().numpy()
         assert np.array_equal(got[..., 3], ok.astype(np.float32))
         assert np.array_equal(_bits(got[..., :3][ok != 0]), _bits(want[ok != 0]))
+
+
+@pytest.mark.parametrize("form", ["plain", "chosen"])
+@pytest.mark.parametrize("size,stride", [((1, 1), 1), ((7, 9), 1), ((33, 17), 2), ((300, 120), 1), ((304, 129), 1),
+                                         ((97, 61), 3)])
+def test_allocation_of_small_and_large_tiles(env, small_orbit, form, size, stride):
+    """Frames whose filter and allocation run in tiles of 8x4 pixels (up to 152 tiles of 32x8: 300x120 is 10 by 15) and of
+    32x8 (304x129 is 10 by 17): the oracle's blocks and layers, word for word, with both allocation rules; many
+    blocks to a tile (a short focal length)."""
+    backend, O = env
+    from voxelhashmt_gb300 import _capi, scenes
+    on = int(form == "chosen")
+    w, h = size
+    sc = scenes.orbit_scene(seed=7, frames=4, width=w, height=h, fx=0.4 * w, fy=0.4 * w, cx=w / 2.0, cy=h / 2.0)
+    sc.voxel_size, sc.truncation = 0.02, 0.06
+    vol = backend.VoxelHashTSDF(sc.voxel_size, sc.truncation, hash_buckets=1 << 17, max_blocks=16384,
+                                algorithm=_capi.default_algorithm(allocation_mode=on, normal_mode=on))
+    ora = O.Volume(O.config(O.FLAVOR_REF_GPU, O.EXP_OWN, threads=8, alloc_mode=on, normal_mode=on), sc.voxel_size,
+                   sc.truncation)
+    for f in (0, 2):
+        d = scenes.render_depth(sc, f)
+        backend.integrate_depth_frame_cuda(vol, backend.DepthFrame(sc.intrinsics, d), sc.poses[f], stride)
+        ora.integrate(d, sc.intrinsics, sc.poses[f], stride)
+    gk, gv = O.sort_blocks(*vol.export_blocks())
+    ok, ov = O.sort_blocks(*ora.blocks())
+    assert np.array_equal(gk, ok)
+    assert np.array_equal(gv.ravel(), ov.view(np.uint32).ravel())
+    vol.close()
+    ora.close()

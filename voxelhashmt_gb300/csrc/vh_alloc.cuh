@@ -27,7 +27,6 @@ namespace alloc {
 constexpr int kTX = 32;
 constexpr int kTY = 8;
 constexpr int kThreads = kTX * kTY;
-constexpr int kCenterSlots = 1024;  // >= 3 * kThreads centres
 constexpr int kMaxSmemProbes = 64;
 
 __device__ __forceinline__ uint32_t smem_hash(unsigned long long k, int bits) {
@@ -80,13 +79,14 @@ __device__ inline void insert_global(const Volume& V, unsigned long long key, ui
   atomicOr(&V.counters->error, kErrHashFull);
 }
 
-// shared-memory set insert; returns 1 if inserted, 0 if present, -1 if the probe budget ran out.  A slot is read
+// shared-memory set insert; returns 1 if inserted (into `slot`), 0 if present, -1 if the probe budget ran out.  A slot is read
 // before it is exchanged: most samples of a tile bring a key that is there already, and 32 lanes that exchange on one
 // address take turns where 32 reads of it are one (with the stamp check above: 110 -> 104 us a frame in the exact build
 // and 32 -> 31 in the fast-math one, 640x480 room).
-__device__ __forceinline__ int smem_insert(unsigned long long* set, int bits, unsigned long long key) {
+__device__ __forceinline__ int smem_insert(unsigned long long* set, int bits, unsigned long long key, uint32_t& slot) {
   const uint32_t mask = (1U << bits) - 1U;
-  uint32_t s = smem_hash(key, bits);
+  uint32_t& s = slot;
+  s = smem_hash(key, bits);
   for (int probe = 0; probe < kMaxSmemProbes; ++probe) {
     unsigned long long prev = *reinterpret_cast<volatile unsigned long long*>(&set[s]);
     if (prev == key) return 0;
@@ -98,10 +98,52 @@ __device__ __forceinline__ int smem_insert(unsigned long long* set, int bits, un
   return -1;
 }
 
+// Shared-memory sets of one tile of kSamples samples, kT threads.  kBand: the truncation-band rule only
+// (Params::alloc_mode 1), which needs just the tile's key set, and a small one: a tile's band crosses tens of blocks,
+// and a key that finds the set full goes straight to the device table.  klist: the slots of the set's keys, in the order
+// they came, so that the inserts into the device table (each a chain of dependent L2/DRAM round trips) run one per
+// thread and none after another, without a search of the sparse set.
+template <bool kBand, int kSamples, int kT, int kBits>
+struct Sets;
+template <int kSamples, int kT, int kBits>
+struct Sets<false, kSamples, kT, kBits> {
+  static constexpr int kThreads = kT, kSetBits = kBits, kCenterBits = kSamples > 128 ? 10 : 8;
+  static_assert((1 << kCenterBits) >= 3 * kSamples, "three centres a sample");
+  unsigned long long clist[3 * kSamples];
+  unsigned long long nset[1 << kBits];
+  union {
+    unsigned long long cset[1 << kCenterBits];  // while the centres are collected
+    uint16_t klist[1 << kBits];                 // from then on
+  };
+  uint32_t ccount, nkeys;
+};
+template <int kSamples, int kT, int kBits>
+struct Sets<true, kSamples, kT, kBits> {
+  static constexpr int kThreads = kT, kSetBits = kBits;
+  unsigned long long nset[1 << kBits];
+  uint16_t klist[1 << kBits];
+  uint32_t nkeys;
+};
+template <bool kBand>
+using TileSets = Sets<kBand, alloc::kThreads, alloc::kThreads, kBand ? 10 : 12>;
+using Smem = TileSets<false>;
+
+// a key of the tile: into its set, or straight into the device table when the set is saturated
+template <class S>
+__device__ __forceinline__ void tile_insert(const Volume& V, S& sets, unsigned long long key, uint32_t frame) {
+  uint32_t slot;
+  const int r = smem_insert(sets.nset, S::kSetBits, key, slot);
+  if (r < 0) {
+    insert_global(V, key, frame);
+  } else if (r == 1) {
+    sets.klist[atomicAdd(&sets.nkeys, 1U)] = static_cast<uint16_t>(slot);
+  }
+}
+
 // Blocks crossed by the segment a -> b (3-D DDA over the block grid, Amanatides & Woo 1987), each inserted into
 // the tile set; returns false when a block leaves the packed key range.
-__device__ inline bool insert_band_blocks(const Volume& V, unsigned long long* s_nset, int set_bits, f3 a, f3 b, float bws,
-                                          uint32_t frame) {
+template <class S>
+__device__ __forceinline__ bool insert_band_blocks(const Volume& V, S& sets, f3 a, f3 b, float bws, uint32_t frame) {
   int c[3] = {static_cast<int>(floorf(a.x / bws)), static_cast<int>(floorf(a.y / bws)), static_cast<int>(floorf(a.z / bws))};
   const int e[3] = {static_cast<int>(floorf(b.x / bws)), static_cast<int>(floorf(b.y / bws)),
                     static_cast<int>(floorf(b.z / bws))};
@@ -118,7 +160,7 @@ __device__ inline bool insert_band_blocks(const Volume& V, unsigned long long* s
   for (int it = 0; it < 64; ++it) {
     unsigned long long key;
     if (!pack_block_key(c[0], c[1], c[2], key)) return false;
-    if (smem_insert(s_nset, set_bits, key) < 0) insert_global(V, key, frame);
+    tile_insert(V, sets, key, frame);
     if (c[0] == e[0] && c[1] == e[1] && c[2] == e[2]) break;
     const int k = (tmax[0] < tmax[1]) ? (tmax[0] < tmax[2] ? 0 : 2) : (tmax[1] < tmax[2] ? 1 : 2);
     // the step on axis k, written per axis so that the arrays stay in registers (no indexing by a run-time k)
@@ -134,49 +176,23 @@ __device__ inline bool insert_band_blocks(const Volume& V, unsigned long long* s
   }
   unsigned long long key;  // the end block always belongs to the band (the set drops the duplicate)
   if (!pack_block_key(e[0], e[1], e[2], key)) return false;
-  if (smem_insert(s_nset, set_bits, key) < 0) insert_global(V, key, frame);
+  tile_insert(V, sets, key, frame);
   return true;
 }
 
-// Shared-memory sets of one tile.  kBand: the truncation-band rule only (Params::alloc_mode 1), which needs
-// just the tile's key set, and a small one: a tile's band crosses tens of blocks, and a key that finds the set
-// full goes straight to the device table.
-template <bool kBand>
-struct TileSets;
-template <>
-struct TileSets<false> {
-  static constexpr int kSetBits = 12;
-  unsigned long long cset[kCenterSlots];
-  unsigned long long clist[3 * kThreads];
-  unsigned long long nset[1 << kSetBits];
-  uint32_t ccount;
-};
-template <>
-struct TileSets<true> {
-  static constexpr int kSetBits = 10;
-  unsigned long long nset[1 << kSetBits];
-  unsigned long long klist[1 << kSetBits];  // the set's keys, compacted
-  uint32_t nkeys;
-};
-using Smem = TileSets<false>;
-
-// buildActiveBlockHashKernel (cuda_block_allocator.cu:231-272) for one tile of kThreads samples; every thread
-// of the CTA calls it (it synchronises).  Thread tid holds one sample: has = it exists and lies in the image,
-// (u, v) its pixel, d its depth.  kBand = false runs the rule p.alloc_mode selects; kBand = true requires
-// p.alloc_mode == 1.
-template <bool kBand>
+// buildActiveBlockHashKernel (cuda_block_allocator.cu:231-272) for one tile; every thread of the CTA calls it (it
+// synchronises).  Thread tid holds one sample: has = it exists and lies in the image, (u, v) its pixel, d its depth.
+// kBand = false runs the rule p.alloc_mode selects; kBand = true requires p.alloc_mode == 1.
+template <bool kBand, int kSamples, int kT, int kBits>
 __device__ __forceinline__ void alloc_samples(const Volume& V, const Params& p, bool has, int u, int v, float d, int tid,
-                                              TileSets<kBand>& S) {
-  constexpr int kSetBits = TileSets<kBand>::kSetBits;
-  unsigned long long* s_nset = S.nset;
+                                              Sets<kBand, kSamples, kT, kBits>& S) {
   const uint32_t frame = V.counters->frame;
-  for (int i = tid; i < (1 << kSetBits); i += kThreads) s_nset[i] = kEmptyKey;
+  for (int i = tid; i < (1 << kBits); i += kT) S.nset[i] = kEmptyKey;
   if constexpr (!kBand) {
-    for (int i = tid; i < kCenterSlots; i += kThreads) S.cset[i] = kEmptyKey;
+    for (int i = tid; i < (1 << S.kCenterBits); i += kT) S.cset[i] = kEmptyKey;
     if (tid == 0) S.ccount = 0U;
-  } else {
-    if (tid == 0) S.nkeys = 0U;
   }
+  if (tid == 0) S.nkeys = 0U;
   __syncthreads();
 
   // 1. centre blocks of this sample (buildActiveBlockHashKernel, cuda_block_allocator.cu:231-272)
@@ -190,7 +206,7 @@ __device__ __forceinline__ void alloc_samples(const Volume& V, const Params& p, 
         mk3(pw.x + ray.x * p.truncation, pw.y + ray.y * p.truncation, pw.z + ray.z * p.truncation),
     };
     if (kBand || p.alloc_mode == 1) {
-      if (!insert_band_blocks(V, s_nset, kSetBits, pts[1], pts[2], p.block_world_size, frame)) {
+      if (!insert_band_blocks(V, S, pts[1], pts[2], p.block_world_size, frame)) {
         atomicOr(&V.counters->error, kErrKeyRange);
       }
     } else {
@@ -208,7 +224,8 @@ __device__ __forceinline__ void alloc_samples(const Volume& V, const Params& p, 
           }
           unsigned long long key;
           pack_block_key(bx, by, bz, key);
-          const int r = smem_insert(S.cset, 10, key);
+          uint32_t slot;
+          const int r = smem_insert(S.cset, S.kCenterBits, key, slot);
           if (r == 1) {
             const uint32_t pos = atomicAdd(&S.ccount, 1U);
             S.clist[pos] = key;
@@ -228,34 +245,20 @@ __device__ __forceinline__ void alloc_samples(const Volume& V, const Params& p, 
   if constexpr (!kBand) {
     // 2. 27-neighbourhoods of the unique centres (insertNeighborhood, :198-220)
     const int ncent = static_cast<int>(S.ccount);
-    for (int w = tid; w < ncent * 27; w += kThreads) {
+    for (int w = tid; w < ncent * 27; w += kT) {
       const int c = w / 27, o = w - c * 27;
       int x, y, z;
       unpack_block_key(S.clist[c], x, y, z);
       unsigned long long key;
       pack_block_key(x + (o % 3) - 1, y + ((o / 3) % 3) - 1, z + (o / 9) - 1, key);
-      if (smem_insert(s_nset, kSetBits, key) < 0) insert_global(V, key, frame);  // tile set saturated
+      tile_insert(V, S, key, frame);
     }
     __syncthreads();
   }
 
-  // 3. one persistent-hash insert per unique key of the tile.  The band's set is sparse (tens of keys in 1,024
-  // slots): its keys are compacted first, so that every insert (a chain of dependent L2/DRAM round trips) runs
-  // on its own thread at once instead of one after another in the threads that own several set slots.
-  if constexpr (kBand) {
-    for (int s = tid; s < (1 << kSetBits); s += kThreads) {
-      const unsigned long long key = s_nset[s];
-      if (key != kEmptyKey) S.klist[atomicAdd(&S.nkeys, 1U)] = key;
-    }
-    __syncthreads();
-    const int n = static_cast<int>(S.nkeys);
-    for (int i = tid; i < n; i += kThreads) insert_global(V, S.klist[i], frame);
-  } else {
-    for (int s = tid; s < (1 << kSetBits); s += kThreads) {
-      const unsigned long long key = s_nset[s];
-      if (key != kEmptyKey) insert_global(V, key, frame);
-    }
-  }
+  // 3. one persistent-hash insert per unique key of the tile
+  const int n = static_cast<int>(S.nkeys);
+  for (int i = tid; i < n; i += kT) insert_global(V, S.nset[S.klist[i]], frame);
 }
 
 // the tile of samples at (sx0, sy0) (sample (sx, sy) = pixel (sx * stride, sy * stride)), depth from global memory
@@ -265,7 +268,7 @@ __device__ __forceinline__ void alloc_tile(const float* __restrict__ depth, cons
   const int u = sx * p.stride, v = sy * p.stride;
   const bool has = sx < p.sample_width && sy < p.sample_height && u < p.width && v < p.height;
   const float d = has ? __ldg(&depth[static_cast<size_t>(v) * p.width + u]) : 0.0f;
-  alloc_samples<false>(V, p, has, u, v, d, tid, S);
+  alloc_samples(V, p, has, u, v, d, tid, S);
 }
 
 }  // namespace alloc

@@ -626,5 +626,10 @@ inline cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 b
 // 68 and 33, 480x360 (675) 73 and 65, 640x480 (1,200) 103 and 109, 1280x960 347 and 404 (the small tiles' halo is
 // three times their area, the large ones' 1.7).  The normal map of the fast-math build crosses at the same size.
 inline bool few_tiles(dim3 large) { return static_cast<unsigned long long>(large.x) * large.y <= 6ULL * 152ULL; }
+// The filter with the allocation (filter_alloc_small_kernel): at most one large tile per SM.  A smaller tile finds more of
+// its blocks found by its neighbours too, and each goes to the device table again: large and small (us), exact build
+// 160x120 36 and 15, 320x240 32 and 35, 480x360 51 and 67; fast-math build with the band rule 160x120 16 and 10,
+// 320x240 16 and 14 (orbit) or 17 and 26 (room).
+inline bool very_few_tiles(dim3 large) { return static_cast<unsigned long long>(large.x) * large.y <= 152ULL; }
 
 }  // namespace vh

@@ -114,7 +114,6 @@ __device__ __forceinline__ void bilateral_taps(const Smem& S, int tx, int ty, fl
   }
 }
 
-#ifndef VH_FAST_MATH
 // The filter of a small image: a tile of 8x4 pixels, and each of its up to 25 taps' weights computed by a warp of its
 // own lanes (lane = pixel) into shared memory; one warp then adds them in the reference's order.  With 32x8 tiles and
 // a thread per pixel an image of 160x120 is 75 CTAs of 25 taps with two exponentials each, one after another: the time
@@ -125,10 +124,12 @@ struct SmallSmem {
   float depth[kSmallTY + 2 * (kR + 1)][kSmallTX + 2 * (kR + 1)];
   float4 normal[kSmallTY + 2 * kR][kSmallTX + 2 * kR];
   float spatial[(2 * kR + 1) * (2 * kR + 1)];
-  float2 tap[(2 * kR + 1) * (2 * kR + 1)][kSmallTX * kSmallTY];  // weight * depth, weight
+  float2 tap[(2 * kR + 1) * (2 * kR + 1)][kSmallTX * kSmallTY];  // depth and weight, zeros for a tap left out
 };
 
-__device__ __forceinline__ void filter_small_tile(const float* __restrict__ in, float* __restrict__ out,
+// every thread of the CTA calls it; thread t < 32 writes pixel (u0 + t % 8, v0 + t / 8) and returns the value (0 outside
+// the image)
+__device__ __forceinline__ float filter_small_tile(const float* __restrict__ in, float* __restrict__ out,
                                                   const Params& p, int u0, int v0, int tid, SmallSmem& S) {
   constexpr int kW = kSmallTX + 2 * (kR + 1), kH = kSmallTY + 2 * (kR + 1);
   constexpr int kNx = kSmallTX + 2 * kR, kNy = kSmallTY + 2 * kR;
@@ -160,34 +161,56 @@ __device__ __forceinline__ void filter_small_tile(const float* __restrict__ in, 
   for (int k = tid >> 5; k < taps; k += kSmallThreads / 32) {
     const int dv = k / side - p.filter_radius, du = k % side - p.filter_radius;
     const float sd = S.depth[ty + kR + 1 + dv][tx + kR + 1 + du];
-    float w = 0.0f, wd = 0.0f;
+    float2 t = make_float2(0.0f, 0.0f);
     const float delta = sd - center;
     const float range = delta * delta;
-    if (center > 0.0f && !(sd <= 0.0f) && !(fabsf(delta) > thr) && !gaussian_is_zero(range, p.filter_k_range)) {
+    bool in = center > 0.0f && !(sd <= 0.0f) && !(fabsf(delta) > thr);
+#ifndef VH_FAST_MATH
+    in = in && !gaussian_is_zero(range, p.filter_k_range);  // adds zeros
+#endif
+    if (in) {
       const float4 sn = S.normal[ty + kR + dv][tx + kR + du];
-      const float cosine = clampf(dot3(mk3(cn4.x, cn4.y, cn4.z), mk3(sn.x, sn.y, sn.z)), -1.0f, 1.0f);
+#ifdef VH_FAST_MATH
+      // the fused multiply-adds that the compiler makes of bilateral_taps, written out: the same depth for either tile
+      const float dot = __fmaf_rn(cn4.z, sn.z, __fmaf_rn(cn4.y, sn.y, __fmul_rn(cn4.x, sn.x)));
+#else
+      const float dot = dot3(mk3(cn4.x, cn4.y, cn4.z), mk3(sn.x, sn.y, sn.z));
+#endif
+      const float cosine = clampf(dot, -1.0f, 1.0f);
+      const float ad = 1.0f - cosine;
       if (!has_cn || (sn.w != 0.0f && !(cosine < p.filter_min_cos))) {
-        w = S.spatial[(dv + kR) * (2 * kR + 1) + (du + kR)] * gaussian(range, p.filter_k_range);
-        const float ad = 1.0f - cosine;
+#ifdef VH_FAST_MATH
+        float e = __fmul_rn(range, p.filter_k_range);
+        if (has_cn) e = __fmaf_rn(__fmul_rn(ad, ad), p.filter_k_angular, e);
+        const float w = __fmul_rn(S.spatial[(dv + kR) * (2 * kR + 1) + (du + kR)], __expf(-e));
+#else
+        float w = S.spatial[(dv + kR) * (2 * kR + 1) + (du + kR)] * gaussian(range, p.filter_k_range);
         if (has_cn) w *= gaussian(ad * ad, p.filter_k_angular);
-        wd = w * sd;
+#endif
+        t = make_float2(sd, w);
       }
     }
-    S.tap[k][lane] = make_float2(wd, w);
+    S.tap[k][lane] = t;
   }
   __syncthreads();
   const int u = u0 + tx, v = v0 + ty;
-  if (tid >= 32 || u >= p.width || v >= p.height) return;
+  if (tid >= 32 || u >= p.width || v >= p.height) return 0.0f;
   float wds = 0.0f, ws = 0.0f;  // a tap left out adds zeros
 #pragma unroll 5
   for (int k = 0; k < taps; ++k) {
     const float2 t = S.tap[k][lane];
-    wds += t.x;
+#ifdef VH_FAST_MATH
+    wds = __fmaf_rn(t.y, t.x, wds);
+    ws = __fadd_rn(ws, t.y);
+#else
+    wds += t.y * t.x;
     ws += t.y;
-  }
-  out[static_cast<size_t>(v) * p.width + u] = center <= 0.0f ? 0.0f : (ws > 1e-6f ? wds / ws : center);
-}
 #endif
+  }
+  const float result = center <= 0.0f ? 0.0f : (ws > 1e-6f ? wds / ws : center);
+  out[static_cast<size_t>(v) * p.width + u] = result;
+  return result;
+}
 
 // bilateralFilterDepthKernel (cuda_tsdf_integrator.cu:650-725) for the output tile at (u0, v0); every thread of
 // the CTA calls it (it synchronises); thread (tx, ty) = tid % kTX, tid / kTX writes pixel (u0 + tx, v0 + ty)

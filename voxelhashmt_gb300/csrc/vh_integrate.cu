@@ -27,6 +27,8 @@
 // The file is compiled twice: as vh::exact (the bit-reproducible FP32 form: -fmad=false, IEEE division and
 // square root, vh_expf) and, with VH_FAST_MATH, as vh::fast (fused multiply-adds, approximate division, square
 // root and exponential; selected per volume by vh_algorithm.fast_math).
+#include <type_traits>
+
 #include "vh_alloc.cuh"
 #include "vh_common.cuh"
 #include "vh_filter.cuh"
@@ -993,18 +995,21 @@ __global__ void __launch_bounds__(kMapTX * kMapTY) pixel_normal_kernel(const flo
   map_tile(depth, p, nmap, blockIdx.x * kMapTX, blockIdx.y * kMapTY, threadIdx.y * kMapTX + threadIdx.x, S);
 }
 
-// The normal map of a frame (pixel_normal_kernel) plus, grid-stride over the frame's visible list (final: the
-// allocation ran before), each entry's {block key, pool index} into V.visible_keys, so that the fused update
-// reads one int4 per chunk instead of the dependent chain visible -> slot_block -> block_keys.
-__global__ void __launch_bounds__(kMapTX * kMapTY) map_prepare_kernel(const float* __restrict__ depth, const Volume V,
-                                                                      const Params p, float4* __restrict__ nmap) {
-  __shared__ MapSmem S;
-  const int tid = threadIdx.y * kMapTX + threadIdx.x;
+// The normal map of a frame (pixel_normal_kernel, or pixel_normal_small_kernel for a small image) plus, grid-stride over
+// the frame's visible list (final: the allocation ran before), each entry's {block key, pool index} into
+// V.visible_keys, so that the fused update reads one int4 per chunk instead of the dependent chain visible ->
+// slot_block -> block_keys.
+template <bool kSmall>
+__global__ void __launch_bounds__(kSmall ? kSmallMapThreads : kMapTX * kMapTY)
+    map_prepare_kernel(const float* __restrict__ depth, const Volume V, const Params p, float4* __restrict__ nmap) {
+  __shared__ std::conditional_t<kSmall, SmallMapSmem, MapSmem> S;
+  constexpr int kT = kSmall ? kSmallMapThreads : kMapTX * kMapTY;
+  const int tid = threadIdx.x;
   allow_next();
   wait_previous();
   const uint32_t nvis = V.counters->visible_count;
-  const uint32_t nthreads = gridDim.x * gridDim.y * kMapTX * kMapTY;
-  for (uint32_t i = (blockIdx.y * gridDim.x + blockIdx.x) * (kMapTX * kMapTY) + tid; i < nvis; i += nthreads) {
+  const uint32_t nthreads = gridDim.x * gridDim.y * kT;
+  for (uint32_t i = (blockIdx.y * gridDim.x + blockIdx.x) * kT + tid; i < nvis; i += nthreads) {
     const uint32_t b = V.slot_block[V.visible[i]];
     int4 k = make_int4(0, 0, 0, static_cast<int>(kInvalidBlock));
     if (b != kInvalidBlock) {
@@ -1013,7 +1018,11 @@ __global__ void __launch_bounds__(kMapTX * kMapTY) map_prepare_kernel(const floa
     }
     V.visible_keys[i] = k;
   }
-  map_tile(depth, p, nmap, blockIdx.x * kMapTX, blockIdx.y * kMapTY, tid, S);
+  if constexpr (kSmall) {
+    map_tile_small(depth, p, nmap, blockIdx.x * kSmallMapTX, blockIdx.y * kSmallMapTY, tid, S);
+  } else {
+    map_tile(depth, p, nmap, blockIdx.x * kMapTX, blockIdx.y * kMapTY, tid, S);
+  }
 }
 
 // Normal at a voxel's projection (u, v): bilinear blend of the valid map taps around it, renormalised.
@@ -1308,7 +1317,7 @@ __device__ __forceinline__ void batch_filter_alloc_body(const SceneDesc* __restr
     const int st = D.p.stride;
     const bool has = u < D.p.width && v < D.p.height && u % st == 0 && v % st == 0 && u / st < D.p.sample_width &&
                      v / st < D.p.sample_height;
-    alloc::alloc_samples<kBand>(D.V, D.p, has, u, v, d, tid, S.a);
+    alloc::alloc_samples(D.V, D.p, has, u, v, d, tid, S.a);
     __syncthreads();
   }
 }
@@ -1635,7 +1644,29 @@ __global__ void __launch_bounds__(filt::kTX * filt::kTY) filter_alloc_kernel(con
   const int u = u0 + tid % filt::kTX, v = v0 + tid / filt::kTX;
   const bool has = u < p.width && v < p.height && u % p.stride == 0 && v % p.stride == 0 &&
                    u / p.stride < p.sample_width && v / p.stride < p.sample_height;
-  alloc::alloc_samples<kBand>(V, p, has, u, v, d, tid, S.a);
+  alloc::alloc_samples(V, p, has, u, v, d, tid, S.a);
+}
+
+// The same for a small image (very_few_tiles): tiles of 8x4 pixels, the filter's taps spread over the CTA's warps
+// (filter_small_tile), the 32 samples allocated by the CTA.
+template <bool kBand>
+__global__ void __launch_bounds__(filt::kSmallThreads) filter_alloc_small_kernel(const float* __restrict__ in,
+                                                                                 float* __restrict__ out, const Volume V,
+                                                                                 const Params p) {
+  __shared__ union Shared {
+    filt::SmallSmem f;
+    alloc::Sets<kBand, 32, filt::kSmallThreads, kBand ? 8 : 10> a;
+  } S;
+  const int tid = threadIdx.x;
+  const int u0 = blockIdx.x * filt::kSmallTX, v0 = blockIdx.y * filt::kSmallTY;
+  allow_next();
+  const float d = filt::filter_small_tile(in, out, p, u0, v0, tid, S.f);
+  __syncthreads();
+  wait_previous();
+  const int u = u0 + tid % filt::kSmallTX, v = v0 + tid / filt::kSmallTX;
+  const bool has = tid < 32 && u < p.width && v < p.height && u % p.stride == 0 && v % p.stride == 0 &&
+                   u / p.stride < p.sample_width && v / p.stride < p.sample_height;
+  alloc::alloc_samples(V, p, has, u, v, d, tid, S.a);
 }
 
 }  // namespace
@@ -1666,6 +1697,11 @@ cudaError_t launch_filter_alloc(const float* in, float* out, const Volume& V, co
   const cudaError_t e = launch_begin_frame(V.counters, s);
   if (e != cudaSuccess) return e;
   const dim3 grid((p.width + filt::kTX - 1) / filt::kTX, (p.height + filt::kTY - 1) / filt::kTY);
+  if (very_few_tiles(grid)) {
+    const dim3 small((p.width + filt::kSmallTX - 1) / filt::kSmallTX, (p.height + filt::kSmallTY - 1) / filt::kSmallTY);
+    return launch_dependent(p.alloc_mode == 1 ? filter_alloc_small_kernel<true> : filter_alloc_small_kernel<false>, small,
+                            dim3(filt::kSmallThreads), s, in, out, V, p);
+  }
   return launch_dependent(p.alloc_mode == 1 ? filter_alloc_kernel<true> : filter_alloc_kernel<false>, grid,
                           dim3(filt::kTX * filt::kTY), s, in, out, V, p);
 }
@@ -1685,8 +1721,12 @@ cudaError_t launch_integrate_prepare(const float* depth, const Volume& V, const 
                                      cudaStream_t s) {
   if (p.normal_mode == 1) {
     if (nmap == nullptr) return cudaErrorInvalidValue;
-    const dim3 mb(kMapTX, kMapTY), mg((p.width + kMapTX - 1) / kMapTX, (p.height + kMapTY - 1) / kMapTY);
-    return launch_dependent(map_prepare_kernel, mg, mb, s, depth, V, p, nmap);
+    const dim3 mg((p.width + kMapTX - 1) / kMapTX, (p.height + kMapTY - 1) / kMapTY);
+    if (few_tiles(mg)) {
+      const dim3 small((p.width + kSmallMapTX - 1) / kSmallMapTX, (p.height + kSmallMapTY - 1) / kSmallMapTY);
+      return launch_dependent(map_prepare_kernel<true>, small, kSmallMapThreads, s, depth, V, p, nmap);
+    }
+    return launch_dependent(map_prepare_kernel<false>, mg, kMapTX * kMapTY, s, depth, V, p, nmap);
   }
   static int classify_grid = 0;
   if (classify_grid == 0) classify_grid = grid_for(reinterpret_cast<const void*>(classify_kernel), kThreads);
