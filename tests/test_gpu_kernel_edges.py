@@ -112,6 +112,47 @@ def _random_blocks(rng, keys, vs, fill):
 
 
 @pytest.mark.parametrize("fp16", [0, 1])
+def test_export_and_reset_by_stored_directions(env, small_orbit, fp16):
+    """Blocks with layers in no, one, several and all directions, and with a direction of records without weight alone (kept
+    word for word by FP32 storage, empty in FP16): exported as they were imported; a reset leaves nothing of them."""
+    backend, O = env
+    from voxelhashmt_gb300 import _capi, scenes
+    sc, vs = small_orbit, small_orbit.voxel_size
+    rng = np.random.default_rng(11)
+    keys = np.array([(x, y, 0) for y in range(40) for x in range(40)], np.int32)  # more than the clearing CTAs
+    vox = _random_blocks(rng, keys, vs, 0.05)
+    dirs = rng.integers(0, 64, len(keys))
+    dirs[:3] = (0, 1, 63)
+    vox[((dirs[:, None] >> np.arange(6)) & 1 == 0)[:, None, :].repeat(512, 1)] = 0
+    stray = (dirs >> 3) & 1 == 0
+    vox[stray, 7, 3, 1, 2] = 0x3f800000  # a plane offset without a weight
+    vol, fresh = (backend.VoxelHashTSDF(vs, sc.truncation, hash_buckets=1 << 16, max_blocks=8192, layer_format=fp16)
+                  for _ in range(2))
+    vol.import_blocks(keys, vox)
+    gk, gv = O.sort_blocks(*vol.export_blocks())
+    want = vox.copy()
+    if fp16:
+        want[stray, 7, 3, 1, 2] = 0
+    wk, wv = O.sort_blocks(keys, want)
+    gv, wv = (np.ascontiguousarray(a).view(np.uint32).reshape(len(keys), 512, 6, 3, 4) for a in (gv, wv))
+    assert np.array_equal(gk, wk)
+    if fp16:  # rounded to binary16: the same records observed, the others empty
+        seen = wv[..., 0] != 0
+        assert np.array_equal(gv[..., 0] != 0, seen) and not gv[~seen].any()
+    else:
+        assert np.array_equal(gv, wv)
+    vol.reset()
+    for v in (vol, fresh):
+        for f in (0, 5, 10):
+            backend.integrate_depth_frame_cuda(v, backend.DepthFrame(sc.intrinsics, scenes.render_depth(sc, f)), sc.poses[f])
+    (k1, v1), (k2, v2) = (O.sort_blocks(*v.export_blocks()) for v in (vol, fresh))
+    assert len(k1) > 0 and np.array_equal(k1, k2) and np.array_equal(v1, v2)
+    assert vol.observed_voxel_count() == fresh.observed_voxel_count() == vol.recount_observed_voxels()
+    vol.close()
+    fresh.close()
+
+
+@pytest.mark.parametrize("fp16", [0, 1])
 @pytest.mark.parametrize("fill,iso", [(0.02, 0.0), (0.35, 0.0), (0.9, 0.004)])
 def test_mesh_of_random_layers(env, fp16, fill, iso):
     """Marching cubes of blocks of random planes against the oracle: from nearly empty blocks to every cell marked in

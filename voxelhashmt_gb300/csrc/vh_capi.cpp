@@ -672,7 +672,7 @@ vh_status vh_reset(vh_volume* v, void* stream) {
   VH_CUDA(v, cudaMemsetAsync(V.slot_keys, 0xFF, V.capacity * sizeof(unsigned long long), s));
   VH_CUDA(v, cudaMemsetAsync(V.slot_block, 0xFF, V.capacity * sizeof(uint32_t), s));
   VH_CUDA(v, cudaMemsetAsync(V.slot_stamp, 0, V.capacity * sizeof(uint32_t), s));
-  VH_CUDA(v, cudaMemsetAsync(pool_base(v), 0, used * pool_block_bytes(v), s));
+  VH_CUDA(v, vh::launch_clear_blocks(V, static_cast<uint32_t>(used), s));
   VH_CUDA(v, cudaMemsetAsync(V.obs_mask, 0, used * (vh::kBlockVoxels / 32) * sizeof(uint32_t), s));
   VH_CUDA(v, cudaMemsetAsync(V.dir_mask, 0, used * sizeof(uint32_t), s));
   VH_CUDA(v, cudaMemsetAsync(V.block_stamp, 0, used * sizeof(uint32_t), s));

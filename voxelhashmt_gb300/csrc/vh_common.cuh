@@ -57,7 +57,8 @@ static_assert(sizeof(Counters) == 64, "Counters is read back as one 64-byte copy
 //                                       same dominant direction reads/writes 32 x 48 contiguous bytes
 //   block_keys  int4[max_blocks]        {x, y, z, frame the block was allocated in}
 //   obs_mask    u32[max_blocks][16]     one bit per voxel: any layer observed
-//   dir_mask    u32[max_blocks]         bit d set once any voxel of the block has an observed layer in bin d
+//   dir_mask    u32[max_blocks]         bit d set once anything was stored in direction d of the block (a layer, or an
+//                                       imported record's words): without it the direction is all zeros
 //   visible     u32[capacity]           slots touched by the current frame (unordered)
 //   visible_keys int4[capacity]         per visible entry {x, y, z, pool index}: written after the allocation
 //                                       by the normal-map pass, read once per chunk by the fused update

@@ -232,12 +232,21 @@ __global__ void __launch_bounds__(256) restore_native_kernel(const Volume V, con
     const uint4* from = in + static_cast<size_t>(i) * words;
     for (size_t w = threadIdx.x; w < words; w += blockDim.x) to[w] = from[w];
     __syncthreads();
-    // observed mask and direction mask from the copied bins
+    // observed mask, and the directions that hold any word, from the copied bins
     for (int li = threadIdx.x; li < kBlockVoxels; li += blockDim.x) {
       uint32_t dirs = 0U;
-      for (int d = 0; d < kDirs; ++d)
-        if (bin_observed(V, b, d, li)) dirs |= 1U << d;
-      const unsigned ballot = __ballot_sync(0xffffffffU, dirs != 0U);
+      bool observed = false;
+      for (int d = 0; d < kDirs; ++d) {
+        if (bin_observed(V, b, d, li)) observed = true;
+        uint32_t any = 0U;
+        const size_t bin = words / kDirs / kBlockVoxels;  // 16-byte words of a bin
+        for (size_t w = 0; w < bin; ++w) {
+          const uint4 q = to[(static_cast<size_t>(d) * kBlockVoxels + li) * bin + w];
+          any |= q.x | q.y | q.z | q.w;
+        }
+        if (any) dirs |= 1U << d;
+      }
+      const unsigned ballot = __ballot_sync(0xffffffffU, observed);
       if ((li & 31) == 0) V.obs_mask[static_cast<size_t>(b) * (kBlockVoxels / 32) + (li >> 5)] = ballot;
       if (dirs) atomicOr(&V.dir_mask[b], dirs);
     }

@@ -88,6 +88,8 @@ cudaError_t launch_mc_emit(const Volume& V, const Params& p, const MeshBuffers& 
 cudaError_t launch_recount(const Volume& V, unsigned long long* out, cudaStream_t s);
 // keys of the current frame's visible blocks (int3 each, unordered)
 cudaError_t launch_visible_keys(const Volume& V, int* keys, cudaStream_t s);
+// zeros into the stored directions of blocks [0, count): their bins are then all zeros
+cudaError_t launch_clear_blocks(const Volume& V, uint32_t count, cudaStream_t s);
 // copy blocks [first, first+count), or the listed ones (list: count pool indices), to the reference layout: keys
 // int32[count][3], voxels [count][512][6][3] x {f32 weight, f32 surface_coord, f32 plane_offset, u32 packed_normal};
 // either may be null
