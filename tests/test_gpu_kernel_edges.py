@@ -327,3 +327,48 @@ def test_allocation_of_small_and_large_tiles(env, small_orbit, form, size, strid
     assert np.array_equal(gv.ravel(), ov.view(np.uint32).ravel())
     vol.close()
     ora.close()
+
+
+@pytest.mark.parametrize("form", ["plain", "chosen"])
+def test_incremental_mesh_is_every_triangle_of_its_blocks(env, small_orbit, form):
+    """vh_extract_mesh_recent gives all triangles of the full extraction whose cells belong to the blocks of the last frames,
+    and no others: as a volume's first extraction on a stream of its own with the default stream busy, again with
+    the next epochs and two frames, and after a full extraction.  A triangle lies in its cell, so its centroid tells
+    the cell unless it is within rounding of the cell's border (those may be of either)."""
+    from collections import Counter
+    backend, O = env
+    from voxelhashmt_gb300 import _capi, scenes
+    sc, on = small_orbit, int(form == "chosen")
+    vol = backend.VoxelHashTSDF(sc.voxel_size, sc.truncation, hash_buckets=1 << 16, max_blocks=8192, layer_format=on,
+                                algorithm=_capi.default_algorithm(allocation_mode=on, normal_mode=on))
+    stream = torch.cuda.Stream()
+    visible = []
+
+    def integrate(f):
+        backend.integrate_depth_frame_cuda(vol, backend.DepthFrame(sc.intrinsics, scenes.render_depth(sc, f)), sc.poses[f])
+        visible.append({tuple(k) for k in backend.visible_block_keys(vol)})
+
+    def check(recent, frames):
+        full = backend.extract_mesh_cuda(vol)
+        listed = set().union(*visible[-frames:])
+        g = full.reshape(-1, 3, 3).astype(np.float64).mean(1) / sc.voxel_size - 0.5
+        near = (np.abs(g - np.round(g)) < 1e-3).any(1)
+        inside = np.array([tuple(b) in listed for b in np.floor(g).astype(np.int64) >> 3])
+        rows = [r.tobytes() for r in np.ascontiguousarray(full).reshape(len(g), -1)]
+        got = Counter(r.tobytes() for r in np.ascontiguousarray(recent).reshape(len(recent), -1))
+        must = Counter(r for r, i, n in zip(rows, inside, near) if i and not n)
+        may = must + Counter(r for r, n in zip(rows, near) if n)
+        assert 1000 < sum(must.values()) and sum(may.values()) < len(rows) and near.sum() < 0.05 * len(rows)
+        assert not must - got and not got - may
+
+    for f in (0, 6, 12, 18):
+        integrate(f)
+    vol.synchronize()
+    torch.cuda._sleep(200_000_000)
+    check(backend.extract_mesh_cuda(vol, recent_frames=1, stream=stream), 1)
+    integrate(9)
+    check(backend.extract_mesh_cuda(vol, recent_frames=1), 1)
+    check(backend.extract_mesh_cuda(vol, recent_frames=2, stream=stream), 2)
+    integrate(3)
+    check(backend.extract_mesh_cuda(vol, recent_frames=1), 1)
+    vol.close()

@@ -393,7 +393,7 @@ void free_mesh(vh_volume* v) {
   dfree(M.queue);
 }
 
-vh_status ensure_mesh(vh_volume* v) {
+vh_status ensure_mesh(vh_volume* v, cudaStream_t s) {
   vh::MeshBuffers& M = v->mc;
   if (M.queue) return VH_OK;
   const size_t n = v->dev.max_blocks;
@@ -408,7 +408,8 @@ vh_status ensure_mesh(vh_volume* v) {
   VH_CUDA(v, dalloc(&M.dir_totals, n * vh::kDirs));
   VH_CUDA(v, dalloc(&M.offsets, n));
   VH_CUDA(v, dalloc(&M.need, n));
-  VH_CUDA(v, cudaMemset(M.need, 0, n * sizeof(uint32_t)));
+  // on the extraction's stream: a clear on the legacy one could land after the stamps of this very call
+  VH_CUDA(v, cudaMemsetAsync(M.need, 0, n * sizeof(uint32_t), s));
   VH_CUDA(v, dalloc(&M.queue, 4));
   return VH_OK;
 }
@@ -1082,7 +1083,7 @@ static vh_status extract(vh_volume* v, float iso, uint32_t frames, size_t* trian
   if (!v || !triangle_count || v->dev.max_blocks == 0) return fail(v, VH_ERR_INVALID_ARGUMENT, "vh_extract_mesh: bad argument");
   DeviceGuard guard(v->params.device);
   const cudaStream_t s = as_stream(stream);
-  const vh_status st = ensure_mesh(v);
+  const vh_status st = ensure_mesh(v, s);
   if (st != VH_OK) return st;
   const uint32_t* list = nullptr;
   const uint32_t* list_count = nullptr;
