@@ -372,3 +372,51 @@ def test_incremental_mesh_is_every_triangle_of_its_blocks(env, small_orbit, form
     integrate(3)
     check(backend.extract_mesh_cuda(vol, recent_frames=1), 1)
     vol.close()
+
+
+@pytest.mark.parametrize("zero", [("filter_sigma_spatial",), ("filter_sigma_range",), ("filter_sigma_angular",),
+                                  ("normal_sigma_spatial",), ("normal_sigma_range",), ("normal_sigma_angular",),
+                                  ("filter_sigma_range", "filter_sigma_angular", "normal_sigma_range", "normal_sigma_angular"), ()])
+def test_sigmas_of_zero_and_infinite_depth(env, small_orbit, zero):
+    """Sums that are no numbers: a sigma of 0 (its factor is infinite, and the centre's weight NaN), and an infinite depth that
+    no discontinuity threshold leaves out (a weight of 0 times infinity).  The filtered depth, in small and large tiles,
+    and the fused layers are the oracle's; of a layer whose normal is NaN, the weight and the surface coordinate (the bits of
+    its plane offset and its packed normal depend on the machine's NaN)."""
+    backend, O = env
+    from voxelhashmt_gb300 import _capi, scenes
+    sc = small_orbit
+    ours, oras = {k: 0.0 for k in zero}, {k: 0.0 for k in zero}
+    if not zero:
+        ours, oras = {"depth_discontinuity_base": np.inf}, {"disc_base": np.inf}
+    vol = backend.VoxelHashTSDF(sc.voxel_size, sc.truncation, hash_buckets=1 << 16, max_blocks=8192,
+                                algorithm=_capi.default_algorithm(**ours))
+    cfg = O.config(O.FLAVOR_REF_GPU, O.EXP_OWN, threads=8, **oras)
+    ora = O.Volume(cfg, sc.voxel_size, sc.truncation)
+    for f in (0, 3, 6):
+        d = scenes.render_depth(sc, f)
+        if f == 3:
+            d[10:30, 10:40] = 1.25  # neighbours of equal depth
+        backend.integrate_depth_frame_cuda(vol, backend.DepthFrame(sc.intrinsics, d), sc.poses[f])
+        ora.integrate(d, sc.intrinsics, sc.poses[f])
+        if not zero:
+            d[20, 20] = np.inf
+        for w, h in ((64, 48), (1000, 480)):
+            K = scenes.Intrinsics(w, h, sc.intrinsics.fx, sc.intrinsics.fy, sc.intrinsics.cx, sc.intrinsics.cy)
+            Ki, img = _capi.intrinsics(K), np.zeros((h, w), np.float32)
+            img[:48, :64] = d
+            src, out = torch.from_numpy(img).cuda(), torch.empty((h, w), device="cuda")
+            torch.cuda.synchronize()
+            _capi.check(_capi.lib().vh_filter_depth(vol.handle, C.c_void_p(src.data_ptr()), C.c_void_p(out.data_ptr()),
+                                                    C.byref(Ki), None), vol.handle)
+            vol.synchronize()
+            assert np.array_equal(out.cpu().numpy(), O.filter_depth(cfg, img, K), equal_nan=True), (f, w)
+    gk, gv = O.sort_blocks(*vol.export_blocks())
+    ok, ov = O.sort_blocks(*ora.blocks())
+    assert np.array_equal(gk, ok)
+    got, want = gv.reshape(-1, 4), ov.view(np.uint32).reshape(-1, 4)
+    assert np.array_equal(got[:, :2], want[:, :2])
+    nan = np.isnan(want[:, 2].copy().view(np.float32))
+    assert np.array_equal(np.isnan(got[:, 2].copy().view(np.float32)), nan)
+    assert np.array_equal(got[~nan, 2:], want[~nan, 2:])
+    vol.close()
+    ora.close()

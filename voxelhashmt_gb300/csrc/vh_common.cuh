@@ -372,8 +372,13 @@ __device__ __forceinline__ float gaussian(float sq, float k) { return __expf(-sq
 #else
 __device__ __forceinline__ float gaussian(float sq, float k) { return vh_expf(-sq * k); }
 #endif
-// gaussian(sq, k) is exactly 0: the exponent is below log 2^-150 (false for a NaN)
-__device__ __forceinline__ bool gaussian_is_zero(float sq, float k) { return -sq * k < -0x1.9fe368p6f; }
+// A tap with the range weight gaussian(sq, k) adds zeros to its sums: the exponent is below log 2^-150, and no other factor
+// makes a NaN of the product.  An exponent of -infinity comes of an infinite depth or of a sigma of 0, and
+// a sigma of 0 also gives the infinite k_angular of the angular weight: those taps are summed.
+__device__ __forceinline__ bool adds_zeros(float sq, float k, float k_angular) {
+  const float e = -sq * k;
+  return e < -0x1.9fe368p6f && e >= -3.402823466e38f && fabsf(k_angular) <= 3.402823466e38f;
+}
 __device__ __forceinline__ float disc_threshold(const Params& p, float ref) {
   return fmaxf(p.disc_base, p.disc_rel * fmaxf(ref, 0.0f));
 }

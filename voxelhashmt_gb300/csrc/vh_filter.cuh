@@ -97,7 +97,7 @@ __device__ __forceinline__ void bilateral_taps(const Smem& S, int tx, int ty, fl
       }
       const float w = S.spatial[(dv + kR) * (2 * kR + 1) + (du + kR)] * __expf(-e);
 #else
-      if (gaussian_is_zero(range, p.filter_k_range)) continue;  // adds zeros
+      if (adds_zeros(range, p.filter_k_range, p.filter_k_angular)) continue;
       float w = S.spatial[(dv + kR) * (2 * kR + 1) + (du + kR)] * gaussian(range, p.filter_k_range);
       if (has_cn) {
         const float4 sn = S.normal[ty + kR + dv][tx + kR + du];
@@ -166,7 +166,7 @@ __device__ __forceinline__ float filter_small_tile(const float* __restrict__ in,
     const float range = delta * delta;
     bool in = center > 0.0f && !(sd <= 0.0f) && !(fabsf(delta) > thr);
 #ifndef VH_FAST_MATH
-    in = in && !gaussian_is_zero(range, p.filter_k_range);  // adds zeros
+    in = in && !adds_zeros(range, p.filter_k_range, p.filter_k_angular);
 #endif
     if (in) {
       const float4 sn = S.normal[ty + kR + dv][tx + kR + du];

@@ -322,6 +322,7 @@ __device__ __forceinline__ bool surface_normal_fast(const float* __restrict__ de
   f3 cn = mk3(0.0f, 0.0f, 0.0f);
   f3 wsum = cn;
   float ws = 0.0f;
+  const bool range_finite = p.normal_k_range <= 3.402823466e38f;  // not for a sigma of 0: the centre's weight is then NaN
   // the centre's normal (k = -1), then the nine taps: one copy of the normal's and of the exponential's code
 #pragma unroll 1
   for (int k = -1; k < 9; ++k) {
@@ -336,7 +337,7 @@ __device__ __forceinline__ bool surface_normal_fast(const float* __restrict__ de
       const f3 sp = point(s);
       const float delta = sp.z - cp.z;
       range = delta * delta;
-      if (gaussian_is_zero(range, p.normal_k_range)) continue;
+      if (adds_zeros(range, p.normal_k_range, p.normal_k_angular)) continue;
       // estimateSurfaceNormalBaseCamera on the samples, toward the camera
       const f3 cr = cross3(sub3(point(b), point(a)), sub3(point(s + 1), point(s - 1)));
       const float len = norm3(cr);
@@ -362,7 +363,7 @@ __device__ __forceinline__ bool surface_normal_fast(const float* __restrict__ de
     float w = k == 4 ? gs[0] : ((k & 1) ? gs[1] : gs[2]);
     float sq = range, kk = p.normal_k_range;
 #pragma unroll 1
-    for (int e = k == 4 ? 1 : 0; e < 2; ++e) {  // the centre's range weight is 1
+    for (int e = k == 4 && range_finite ? 1 : 0; e < 2; ++e) {  // the centre's range weight is 1
       if (e == 1) {
         sq = ad * ad;
         kk = p.normal_k_angular;
