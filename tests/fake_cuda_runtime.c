@@ -34,8 +34,6 @@ void fake_fail(int copies, int launches_, int attributes) {
 }
 int fake_launches(void) { return launches; }
 int fake_legacy_pending(void) { return legacy_pending; }
-/* a fresh process's view of the kernels */
-void fake_forget_limits(void) { n_limits = 0; }
 
 /* ---- devices, errors ---- */
 err_t cudaGetDeviceCount(int* n) { *n = 2; return 0; }

@@ -80,3 +80,40 @@ def test_work_on_the_legacy_stream_is_waited_for(host, volume):
     assert L.vh_extract_mesh(h, 0.0, C.byref(n), STREAM) == capi.VH_OK
     assert L.vh_reset(h, STREAM) == capi.VH_OK
     assert L.fake_legacy_pending() == 0
+
+
+def _failing_calls(capi, L, h):
+    """name -> (copies, launches, attributes) that fail, and a call that meets them."""
+    K, b, n, f = _intrinsics(capi), _buffer(), C.c_uint64(), C.c_uint32()
+    pose = C.byref(capi.VhPose(R=(C.c_float * 9)(1, 0, 0, 0, 1, 0, 0, 0, 1)))
+    ip = C.cast(b, C.POINTER(C.c_int32))
+    up = C.cast(b, C.POINTER(C.c_uint32))
+    ws = _buffer(L.vh_nn_workspace_bytes(1, 16, 12))
+    return {
+        "copy of a volume's call": ((1, 0, 0), lambda: L.vh_block_count(h, C.byref(n))),
+        "blocks into a buffer": ((1, 0, 0), lambda: L.vh_export_blocks(h, 0, 0, ip, b, 1, STREAM)),
+        "dependent launch": ((0, 1, 0), lambda: L.vh_filter_depth(h, b, b, K, STREAM)),
+        "frame": ((0, 2, 0), lambda: L.vh_integrate(h, b, 1, K, pose, 1, STREAM)),
+        "kernel attribute": ((0, 0, 1), lambda: L.vh_nn_conv32(b, b, None, None, b, 1, 16, 12, 0, 0, up, STREAM)),
+        "tensor-core launch": ((0, 1, 0), lambda: L.vh_nn_conv32(b, b, None, None, b, 1, 16, 12, 0, 0, up, STREAM)),
+        "denoiser": ((0, 2, 0), lambda: L.vh_nn_forward(b, b, b, b, 1, 16, 12, ws, up, STREAM)),
+        "denoiser parameters": ((1, 0, 0), lambda: L.vh_set_depth_denoiser(h, C.cast(b, C.POINTER(C.c_float)))),
+        "exponential check": ((1, 0, 0), lambda: L.vh_expf_check(0, 16, C.byref(n), C.byref(f), STREAM)),
+    }
+
+
+@pytest.mark.parametrize("name", ["copy of a volume's call", "blocks into a buffer", "dependent launch", "frame",
+                                  "kernel attribute", "tensor-core launch", "denoiser", "denoiser parameters",
+                                  "exponential check"])
+def test_a_failed_call_does_not_fail_the_next(host, volume, name):
+    """The error of a call that fails is that call's alone: the next one, on the same volume or on another, succeeds."""
+    capi, L = host
+    h, other = volume(), volume()
+    n = C.c_uint64()
+    fails, call = _failing_calls(capi, L, h)[name]
+    L.fake_fail(*fails)
+    status = call()
+    L.fake_fail(0, 0, 0)
+    assert status == capi.VH_ERR_CUDA
+    for v in (other, h):
+        assert L.vh_recount_observed_voxels(v, C.byref(n), STREAM) == capi.VH_OK

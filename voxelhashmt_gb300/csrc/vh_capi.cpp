@@ -108,9 +108,19 @@ vh_status fail(vh_volume* v, vh_status s, const std::string& msg) {
   return s;
 }
 
+// A call that fails takes its error with it: the runtime keeps the last one, and the launches of the next call, on any
+// volume, would report it as theirs.
 vh_status cuda_fail(vh_volume* v, cudaError_t e, const char* what) {
+  cudaGetLastError();
   const vh_status s = e == cudaErrorMemoryAllocation ? VH_ERR_OUT_OF_MEMORY : VH_ERR_CUDA;
   return fail(v, s, std::string(what) + " failed: " + cudaGetErrorString(e));
+}
+
+// the same for calls without a volume
+vh_status cuda_status(cudaError_t e) {
+  if (e == cudaSuccess) return VH_OK;
+  cudaGetLastError();
+  return VH_ERR_CUDA;
 }
 
 #define VH_CUDA(v, call)                                        \
@@ -505,6 +515,7 @@ vh_status vh_query_device(char* message, size_t len) {
   char buf[256];
   vh_status st = VH_OK;
   if (e != cudaSuccess) {
+    cudaGetLastError();
     std::snprintf(buf, sizeof(buf), "%s", cudaGetErrorString(e));
     st = VH_ERR_NO_DEVICE;
   } else if (count <= 0) {
@@ -530,7 +541,7 @@ vh_status vh_create(const vh_params* params, const vh_algorithm* algo, vh_volume
     return VH_ERR_INVALID_ARGUMENT;  // pool indices are packed with the voxel index in 32 bits
   }
   int count = 0;
-  if (cudaGetDeviceCount(&count) != cudaSuccess || params->device < 0 || params->device >= count) {
+  if (cuda_status(cudaGetDeviceCount(&count)) != VH_OK || params->device < 0 || params->device >= count) {
     return VH_ERR_NO_DEVICE;
   }
   vh_volume* v = new (std::nothrow) vh_volume();
@@ -1334,7 +1345,7 @@ vh_status vh_render_depth(const float* prims, int32_t n_prims, const vh_intrinsi
   for (int i = 0; i < 3; ++i) p.T_wc.t[i] = T_wc->t[i];
   const cudaError_t e = vh::launch_render(prims, n_prims, p, seed, frame, sigma_z2, dropout, max_depth, depth_out,
                                           as_stream(stream));
-  return e == cudaSuccess ? VH_OK : VH_ERR_CUDA;
+  return cuda_status(e);
 }
 
 // ---- multi-scene batch ----
@@ -1437,7 +1448,7 @@ vh_status vh_batch_integrate(vh_batch* b, const float* const* depth_device, cons
   const int slot = b->next;
   b->next ^= 1;
   // the step two calls ago read this staging buffer: wait until it has finished
-  if (cudaEventSynchronize(b->done[slot]) != cudaSuccess) return VH_ERR_CUDA;
+  if (cuda_status(cudaEventSynchronize(b->done[slot])) != VH_OK) return VH_ERR_CUDA;
   auto* hdr = reinterpret_cast<vh::BatchHeader*>(b->h_stage[slot]);
   auto* desc = reinterpret_cast<vh::SceneDesc*>(b->h_stage[slot] + sizeof(vh::BatchHeader));
   const int n = static_cast<int>(b->vols.size());
@@ -1499,9 +1510,7 @@ vh_status vh_batch_integrate(vh_batch* b, const float* const* depth_device, cons
 
 vh_status vh_nn_pack_conv32_weights(const float* w, void* packed, int32_t transpose_flip, void* stream) {
   if (!w || !packed) return VH_ERR_INVALID_ARGUMENT;
-  return vh::nn::launch_pack_w32(w, static_cast<__nv_bfloat16*>(packed), transpose_flip, as_stream(stream)) == cudaSuccess
-             ? VH_OK
-             : VH_ERR_CUDA;
+  return cuda_status(vh::nn::launch_pack_w32(w, static_cast<__nv_bfloat16*>(packed), transpose_flip, as_stream(stream)));
 }
 
 vh_status vh_nn_conv32(const void* in, const void* packed_w, const float* bias, const void* mask, void* out, int32_t batch,
@@ -1514,7 +1523,7 @@ vh_status vh_nn_conv32(const void* in, const void* packed_w, const float* bias, 
                                               static_cast<const __nv_bfloat16*>(packed_w), bias,
                                               static_cast<const __nv_bfloat16*>(mask), static_cast<__nv_bfloat16*>(out),
                                               batch, width, height, mode, relu, error, as_stream(stream));
-  return e == cudaSuccess ? VH_OK : VH_ERR_CUDA;
+  return cuda_status(e);
 }
 
 vh_status vh_nn_conv32_gated(const void* in, const void* packed_w, const float* bias, const void* mask, void* out,
@@ -1528,7 +1537,7 @@ vh_status vh_nn_conv32_gated(const void* in, const void* packed_w, const float* 
                                               static_cast<const __nv_bfloat16*>(packed_w), bias,
                                               static_cast<const __nv_bfloat16*>(mask), static_cast<__nv_bfloat16*>(out),
                                               batch, width, height, mode, relu, error, as_stream(stream), gate);
-  return e == cudaSuccess ? VH_OK : VH_ERR_CUDA;
+  return cuda_status(e);
 }
 
 vh_status vh_nn_wgrad32(const void* x, const void* grad, float* dw, float* db, int32_t batch, int32_t width,
@@ -1537,7 +1546,7 @@ vh_status vh_nn_wgrad32(const void* x, const void* grad, float* dw, float* db, i
   const cudaError_t e = vh::nn::launch_wgrad32(static_cast<const __nv_bfloat16*>(x),
                                                static_cast<const __nv_bfloat16*>(grad), dw, db, batch, width, height,
                                                error, as_stream(stream));
-  return e == cudaSuccess ? VH_OK : VH_ERR_CUDA;
+  return cuda_status(e);
 }
 
 int32_t vh_nn_param_count(void) { return vh::nn::param_count(); }
@@ -1549,8 +1558,7 @@ uint64_t vh_nn_workspace_bytes(int32_t batch, int32_t width, int32_t height) {
 
 vh_status vh_nn_pack(const float* params, void* packed, void* stream) {
   if (!params || !packed) return VH_ERR_INVALID_ARGUMENT;
-  return vh::nn::pack_weights(params, static_cast<__nv_bfloat16*>(packed), as_stream(stream)) == cudaSuccess ? VH_OK
-                                                                                                            : VH_ERR_CUDA;
+  return cuda_status(vh::nn::pack_weights(params, static_cast<__nv_bfloat16*>(packed), as_stream(stream)));
 }
 
 vh_status vh_nn_forward(const float* params, const void* packed, const float* depth, float* out, int32_t batch,
@@ -1558,10 +1566,8 @@ vh_status vh_nn_forward(const float* params, const void* packed, const float* de
   if (!params || !packed || !depth || !out || !workspace || !error || batch <= 0 || width <= 0 || height <= 0) {
     return VH_ERR_INVALID_ARGUMENT;
   }
-  return vh::nn::forward(params, static_cast<const __nv_bfloat16*>(packed), depth, nullptr, out, batch, width, height,
-                         static_cast<unsigned char*>(workspace), error, as_stream(stream)) == cudaSuccess
-             ? VH_OK
-             : VH_ERR_CUDA;
+  return cuda_status(vh::nn::forward(params, static_cast<const __nv_bfloat16*>(packed), depth, nullptr, out, batch,
+                                     width, height, static_cast<unsigned char*>(workspace), error, as_stream(stream)));
 }
 
 vh_status vh_nn_backward(const float* params, const void* packed, const float* depth, const float* target,
@@ -1571,17 +1577,15 @@ vh_status vh_nn_backward(const float* params, const void* packed, const float* d
       width <= 0 || height <= 0) {
     return VH_ERR_INVALID_ARGUMENT;
   }
-  return vh::nn::backward(params, static_cast<const __nv_bfloat16*>(packed), depth, target, out, batch, width, height,
-                          static_cast<unsigned char*>(workspace), grads, loss, error, as_stream(stream)) == cudaSuccess
-             ? VH_OK
-             : VH_ERR_CUDA;
+  return cuda_status(vh::nn::backward(params, static_cast<const __nv_bfloat16*>(packed), depth, target, out, batch,
+                                      width, height, static_cast<unsigned char*>(workspace), grads, loss, error,
+                                      as_stream(stream)));
 }
 
 vh_status vh_nn_adam(float* params, const float* grads, float* m, float* v, float lr, float beta1, float beta2, float eps,
                      int32_t step, void* stream) {
   if (!params || !grads || !m || !v || step < 1) return VH_ERR_INVALID_ARGUMENT;
-  return vh::nn::adam(params, grads, m, v, lr, beta1, beta2, eps, step, as_stream(stream)) == cudaSuccess ? VH_OK
-                                                                                                          : VH_ERR_CUDA;
+  return cuda_status(vh::nn::adam(params, grads, m, v, lr, beta1, beta2, eps, step, as_stream(stream)));
 }
 
 vh_status vh_set_depth_denoiser(vh_volume* v, const float* params) {

@@ -68,7 +68,10 @@ vh_status vh_expf_check(uint32_t first_bits, uint64_t count, uint64_t* mismatche
   if (!mismatches || !first_mismatch || count > (1ULL << 32) - first_bits) return VH_ERR_INVALID_ARGUMENT;
   const cudaStream_t s = static_cast<cudaStream_t>(stream);
   unsigned long long* d = nullptr;
-  if (cudaMalloc(&d, 2 * sizeof(unsigned long long)) != cudaSuccess) return VH_ERR_OUT_OF_MEMORY;
+  if (cudaMalloc(&d, 2 * sizeof(unsigned long long)) != cudaSuccess) {
+    cudaGetLastError();
+    return VH_ERR_OUT_OF_MEMORY;
+  }
   const unsigned long long init[2] = {0ULL, ~0ULL};
   unsigned long long h[2] = {0ULL, ~0ULL};
   cudaError_t e = cudaMemcpyAsync(d, init, sizeof(init), cudaMemcpyHostToDevice, s);
@@ -79,7 +82,10 @@ vh_status vh_expf_check(uint32_t first_bits, uint64_t count, uint64_t* mismatche
   if (e == cudaSuccess) e = cudaMemcpyAsync(h, d, sizeof(h), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   cudaFree(d);
-  if (e != cudaSuccess) return VH_ERR_CUDA;
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return VH_ERR_CUDA;
+  }
   *mismatches = h[0];
   *first_mismatch = h[1] == ~0ULL ? 0xffffffffU : static_cast<uint32_t>(h[1]);
   return VH_OK;
