@@ -117,3 +117,29 @@ def test_a_failed_call_does_not_fail_the_next(host, volume, name):
     assert status == capi.VH_ERR_CUDA
     for v in (other, h):
         assert L.vh_recount_observed_voxels(v, C.byref(n), STREAM) == capi.VH_OK
+
+
+def test_denoiser_on_every_device(host, volume):
+    """The kernels that need more than 48 KB of shared memory are allowed it on each device that runs them, and a refusal is not
+    kept: forward and backward pass and both entry points of a single layer, on the first device, on the second,
+    and after a call that failed."""
+    capi, L = host
+    K, b = (1, 16, 12), _buffer(1 << 20)
+    up, fp = C.cast(b, C.POINTER(C.c_uint32)), b
+    ws = _buffer(L.vh_nn_workspace_bytes(*K))
+    calls = {
+        "forward": lambda: L.vh_nn_forward(fp, b, fp, fp, *K, ws, up, STREAM),
+        "backward": lambda: L.vh_nn_backward(fp, b, fp, fp, fp, *K, ws, fp, fp, up, STREAM),
+        "conv32": lambda: L.vh_nn_conv32(b, b, None, None, b, *K, 0, 0, up, STREAM),
+        "wgrad32": lambda: L.vh_nn_wgrad32(b, b, fp, fp, *K, up, STREAM),
+    }
+    for device in (1, 0, 1):
+        L.cudaSetDevice(device)
+        for name, call in calls.items():
+            L.fake_fail(0, 0, 1)
+            assert call() == capi.VH_ERR_CUDA, (device, name)
+            L.fake_fail(0, 0, 0)
+            before = L.fake_launches()
+            assert call() == capi.VH_OK, (device, name)
+            assert L.fake_launches() > before
+    L.cudaSetDevice(0)

@@ -454,6 +454,21 @@ cudaError_t encode_input_map(const __nv_bfloat16* in, int batch, int width, int 
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
+int sm_count() {
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms > 0 ? sms : 152;
+}
+
+// A kernel's limit of dynamic shared memory is raised on the current device only, and is gone after a reset of that device:
+// it is set before every launch that needs more than 48 KB, not once in the process (a forward pass's three take 0.5-1 us
+// of the 18 us that its launches take on the host).
+template <class Kernel>
+cudaError_t allow_shared(Kernel* kernel, int bytes) {
+  return cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+}
+
 // Launch shapes of conv32_tc_kernel: ring slots, resident CTAs per SM, output rows per block.  Measured on
 // 640x480 layers (CUDA events, batch 1 / batch 16): 6 slots x 2 CTAs x 8 rows 18.7 / 169 us; 8 x 2 x 8
 // 18.7 / 178; 8 x 2 x 16 24.1 / 171; 6 x 3 x 8 18.7 / 219; 4 x 4 x 8 24.8 / 206; the earlier one-row-tile
@@ -490,15 +505,7 @@ cudaError_t launch_conv32(const __nv_bfloat16* in, const __nv_bfloat16* wpack, c
                           int relu, unsigned int* error, cudaStream_t s, const unsigned int* gate) {
   const Conv32Variant& cv = conv32_variant();
   // persistent CTAs, cv.ctas_per_sm per SM: each CTA stages the weights and allocates tensor memory once
-  static int ctas = 0;
-  if (ctas == 0) {
-    cudaError_t e = cudaFuncSetAttribute(cv.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, cv.smem);
-    if (e != cudaSuccess) return e;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    ctas = cv.ctas_per_sm * (sms > 0 ? sms : 152);
-  }
+  const int ctas = cv.ctas_per_sm * sm_count();
   const long long ntiles = static_cast<long long>(batch) * height * ((width + kTile - 1) / kTile);
   if (ntiles > 0x7fffffffLL) return cudaErrorInvalidValue;  // the kernels' tile arithmetic is 32-bit
   const long long nitems =
@@ -506,7 +513,8 @@ cudaError_t launch_conv32(const __nv_bfloat16* in, const __nv_bfloat16* wpack, c
   const int grid = static_cast<int>(nitems < ctas ? nitems : ctas);
   if (grid <= 0) return cudaSuccess;
   CUtensorMap map;
-  const cudaError_t e = encode_input_map(in, batch, width, height, &map);
+  cudaError_t e = encode_input_map(in, batch, width, height, &map);
+  if (e == cudaSuccess) e = allow_shared(cv.fn, cv.smem);
   if (e != cudaSuccess) return e;
   void* args[] = {&map,    const_cast<__nv_bfloat16**>(&wpack), const_cast<float**>(&bias),
                   const_cast<__nv_bfloat16**>(&mask), &out, &batch, &width, &height, &mode, &relu,
@@ -791,22 +799,15 @@ __global__ void __launch_bounds__(kWgThreads, kWgCtasPerSm) wgrad32_tc_kernel(co
 
 cudaError_t launch_wgrad32(const __nv_bfloat16* x, const __nv_bfloat16* g, float* dw, float* db, int batch, int width,
                            int height, unsigned int* error, cudaStream_t s) {
-  static int ctas = 0;
-  if (ctas == 0) {
-    const cudaError_t e =
-        cudaFuncSetAttribute(wgrad32_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgSmem);
-    if (e != cudaSuccess) return e;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    ctas = kWgCtasPerSm * (sms > 0 ? sms : 152);
-  }
+  const int ctas = kWgCtasPerSm * sm_count();
   if (reinterpret_cast<uintptr_t>(x) % 4 != 0 || reinterpret_cast<uintptr_t>(g) % 4 != 0) return cudaErrorInvalidValue;
   const long long nitems = static_cast<long long>(batch) * ((height + kWgRows - 1) / kWgRows) *
                            ((width + kWgStrip - 1) / kWgStrip);
   if (nitems > 0x7fffffffLL) return cudaErrorInvalidValue;  // the item arithmetic is 32-bit
   const int grid = static_cast<int>(nitems < ctas ? nitems : ctas);
   if (grid <= 0) return cudaSuccess;
+  const cudaError_t e = allow_shared(wgrad32_tc_kernel, kWgSmem);
+  if (e != cudaSuccess) return e;
   wgrad32_tc_kernel<<<grid, kWgThreads, kWgSmem, s>>>(x, g, dw, db, batch, width, height, error);
   return cudaGetLastError();
 }
@@ -1429,19 +1430,10 @@ __global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, 
   }
 }
 
-int sm_count();
-
 // CTAs of a tile kernel: at most per_sm resident ones per SM, each taking tiles in turn
 int tile_ctas(int batch, int w, int h, int tw, int th, int per_sm) {
   const long long tiles = tile_grid(batch, w, h, tw, th).count, cap = static_cast<long long>(per_sm) * sm_count();
   return static_cast<int>(tiles < cap ? tiles : cap);
-}
-
-int sm_count() {
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms > 0 ? sms : 152;
 }
 
 }  // namespace
@@ -1492,9 +1484,8 @@ cudaError_t forward(const float* params, const __nv_bfloat16* packed, const floa
     e = launch_conv32(A2, packed + 9 * kC * kC, params + kOffB3, nullptr, A3, batch, width, height, kForward, 1, error, s);
   }
   if (e != cudaSuccess) return e;
-  static const cudaError_t attr =
-      cudaFuncSetAttribute(conv_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kOutSmem);
-  if (attr != cudaSuccess) return attr;
+  e = allow_shared(conv_out_kernel, kOutSmem);
+  if (e != cudaSuccess) return e;
   conv_out_kernel<<<tile_ctas(batch, width, height, kOutW, kOutH, kOutCtas), kTileThreads, kOutSmem, s>>>(
       A3, params, depth, fallback, out, batch, width, height);
   return cudaGetLastError();
@@ -1508,11 +1499,9 @@ cudaError_t backward(const float* params, const __nv_bfloat16* packed, const flo
   carve(ws, n, &A1, &A2, &A3, &G1, &G2);
   cudaError_t e = cudaMemsetAsync(grads, 0, kParams * sizeof(float), s);
   if (e == cudaSuccess) e = cudaMemsetAsync(loss, 0, 2 * sizeof(float), s);
-  if (e != cudaSuccess) return e;
   // the loss, layer 4's weights and the gradient into A3
-  static const cudaError_t attr =
-      cudaFuncSetAttribute(out_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kOutBackSmem);
-  if (attr != cudaSuccess) return attr;
+  if (e == cudaSuccess) e = allow_shared(out_backward_kernel, kOutBackSmem);
+  if (e != cudaSuccess) return e;
   out_backward_kernel<<<tile_ctas(batch, width, height, kTileW, kTileH, 2), kTileThreads, kOutBackSmem, s>>>(
       A3, params, depth, target, out, G1, grads + kOffW4, grads + kOffB4, loss, batch, width, height);
   // layer 3
