@@ -100,7 +100,7 @@ static err_t launch(const void* fn, dim3_t grid, size_t smem) {
     if (limits[i].fn == fn && limits[i].device == device && limits[i].bytes > allowed) allowed = limits[i].bytes;
   }
   if (fail_launches > 0) { --fail_launches; return failed(kInvalidValue); }
-  if (grid.x == 0 || grid.y == 0 || grid.y > 65535 || grid.z != 1 || smem > (size_t)allowed) return failed(kInvalidValue);
+  if (grid.x == 0 || grid.y == 0 || grid.y > 65535 || grid.z == 0 || grid.z > 65535 || smem > (size_t)allowed) return failed(kInvalidValue);
   ++launches;
   return 0;
 }

@@ -420,3 +420,19 @@ def test_sigmas_of_zero_and_infinite_depth(env, small_orbit, zero):
     assert np.array_equal(got[~nan, 2:], want[~nan, 2:])
     vol.close()
     ora.close()
+
+
+@pytest.mark.parametrize("rows", [262140, 262141, 400001])
+def test_raycast_of_a_tall_image(env, small_orbit, rows):
+    """One column of more rows than a grid holds tiles along y (65,535 of 4 rows), against the oracle's ray-cast."""
+    backend, O = env
+    from voxelhashmt_gb300 import scenes
+    sc = small_orbit
+    vol, ora = _fuse(backend, O, sc, [0, 4, 8, 12], 0)
+    K = scenes.Intrinsics(1, rows, 55.4, 55.4 * rows / 48, 0.0, (rows - 1) / 2.0)
+    got = backend.raycast_depth(vol, K, sc.poses[2], 0.0, 3.0, 1.0)
+    want = ora.raycast_depth(K, sc.poses[2], 0.0, 3.0, 1.0)
+    assert (want > 0).sum() > 1000
+    assert np.array_equal(_bits(got), _bits(want))
+    vol.close()
+    ora.close()

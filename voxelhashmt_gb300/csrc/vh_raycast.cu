@@ -34,6 +34,7 @@ namespace vh {
 namespace {
 
 constexpr int kRTX = 8, kRTY = 4;  // pixels per CTA
+constexpr int kMaxGridY = 65535;   // CTAs that a grid holds along y, 262,140 rows: the rest of a taller image goes along z
 constexpr int kRayThreads = 8 * kRTX * kRTY;
 constexpr int kMaxRaySteps = 1 << 16;
 
@@ -135,8 +136,9 @@ __global__ void __launch_bounds__(kRayThreads, 4) raycast_kernel(const Volume V,
   const int px = q & 1, py = (q >> 1) & 1, pz = q >> 2;  // parities of this lane's voxel
   // a warp's four rays are 2x2 pixels, a CTA's eight warps 4x2 of those
   const int warp = ray >> 2, r = ray & 3;
-  const int u = blockIdx.x * kRTX + 2 * (warp & 3) + (r & 1), v = blockIdx.y * kRTY + 2 * (warp >> 2) + (r >> 1);
-  const bool inside = u < p.width && v < p.height;
+  const int u = blockIdx.x * kRTX + 2 * (warp & 3) + (r & 1);
+  const uint32_t v = (blockIdx.z * kMaxGridY + blockIdx.y) * kRTY + 2 * (warp >> 2) + (r >> 1);
+  const bool inside = u < p.width && v < static_cast<uint32_t>(p.height);
   const f3 dc = mk3((static_cast<float>(u) - p.cx) / p.fx, (static_cast<float>(v) - p.cy) / p.fy, 1.0f);
   const f3 dw = xform_vector(p.T_wc, dc);
   const f3 inv_dw = mk3(1.0f / dw.x, 1.0f / dw.y, 1.0f / dw.z);
@@ -253,7 +255,8 @@ __global__ void __launch_bounds__(kRayThreads, 4) raycast_kernel(const Volume V,
 
 cudaError_t launch_raycast(const Volume& V, const Params& p, float min_depth, float max_depth, float step, float* out,
                            cudaStream_t s) {
-  const dim3 grid((p.width + kRTX - 1) / kRTX, (p.height + kRTY - 1) / kRTY);
+  const int ty = (p.height + kRTY - 1) / kRTY;
+  const dim3 grid((p.width + kRTX - 1) / kRTX, ty < kMaxGridY ? ty : kMaxGridY, (ty + kMaxGridY - 1) / kMaxGridY);
   raycast_kernel<<<grid, kRayThreads, 0, s>>>(V, p, min_depth, max_depth, step, out);
   return cudaGetLastError();
 }
