@@ -39,16 +39,15 @@ def host(tmp_path_factory):
 
 @pytest.fixture
 def volume(host):
-    """create(device) -> handle of a small volume; closed at the end."""
+    """create(algorithm options) -> handle of a small volume; closed at the end."""
     capi, L = host
     L.fake_fail(0, 0, 0)
     made = []
 
-    def create(device=0):
+    def create(**algorithm):
         h = C.c_void_p()
         params = capi.default_params(voxel_size=0.02, truncation_distance=0.06, hash_buckets=1 << 10, max_blocks=64)
-        params.device = device
-        assert L.vh_create(C.byref(params), None, C.byref(h)) == capi.VH_OK
+        assert L.vh_create(C.byref(params), C.byref(capi.default_algorithm(**algorithm)), C.byref(h)) == capi.VH_OK
         made.append(h)
         return h
 
@@ -80,6 +79,18 @@ def test_work_on_the_legacy_stream_is_waited_for(host, volume):
     assert L.vh_extract_mesh(h, 0.0, C.byref(n), STREAM) == capi.VH_OK
     assert L.vh_reset(h, STREAM) == capi.VH_OK
     assert L.fake_legacy_pending() == 0
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2])
+def test_a_batch_is_cleared_before_its_first_step(host, volume, mode):
+    """The queue and barrier words of a batch, cleared on the legacy stream, are zero when vh_batch_create returns: a step on
+    a stream that does not wait for the legacy one may follow at once."""
+    capi, L = host
+    vols = (C.c_void_p * 2)(volume(normal_mode=1), volume(normal_mode=1))
+    b = C.c_void_p()
+    assert L.vh_batch_create(vols, 2, mode, C.byref(b)) == capi.VH_OK
+    assert L.fake_legacy_pending() == 0
+    L.vh_batch_destroy(b)
 
 
 def _failing_calls(capi, L, h):

@@ -1426,6 +1426,8 @@ vh_status vh_batch_create(vh_volume* const* volumes, int32_t count, int32_t use_
   cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&b->d_buf), b->bytes);
   if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&b->d_queue), 8 * sizeof(uint32_t));
   if (e == cudaSuccess) e = cudaMemset(b->d_queue, 0, 8 * sizeof(uint32_t));
+  // a step's stream need not wait for the legacy one: the persistent step's barrier words are zero before any step
+  if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
   for (int k = 0; k < 2 && e == cudaSuccess; ++k) {
     e = cudaMallocHost(reinterpret_cast<void**>(&b->h_stage[k]), b->bytes);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->done[k], cudaEventDisableTiming);
