@@ -436,3 +436,36 @@ def test_raycast_of_a_tall_image(env, small_orbit, rows):
     assert np.array_equal(_bits(got), _bits(want))
     vol.close()
     ora.close()
+
+
+@pytest.mark.parametrize("alloc,normal", [(1, 1), (0, 0)])
+def test_fast_math_frames_do_not_depend_on_the_tiles(env, alloc, normal):
+    """The fast-math compile gives a frame the same filtered depth, blocks, layers and normal map, word for word, whether its
+    image is worked on in small tiles (160x120: 75 of 32x8), its filter and allocation in large ones (320x240: 300) or its
+    normal map too (960x360: 1,350).  The frame is the same one, with zeros around it."""
+    backend, O = env
+    from voxelhashmt_gb300 import _capi, scenes
+    w, h = 160, 120
+    sc = scenes.orbit_scene(seed=7, frames=8, width=w, height=h, fx=138.5, fy=138.5, cx=w / 2.0, cy=h / 2.0)
+    sc.voxel_size, sc.truncation = 0.02, 0.06
+    want = None
+    for W, H in ((160, 120), (320, 240), (960, 360)):
+        K = scenes.Intrinsics(W, H, 138.5, 138.5, w / 2.0, h / 2.0)
+        vol = backend.VoxelHashTSDF(sc.voxel_size, sc.truncation, hash_buckets=1 << 16, max_blocks=16384,
+                                    algorithm=_capi.default_algorithm(allocation_mode=alloc, normal_mode=normal, fast_math=1,
+                                                                      autotune=0))
+        Ki, nrm, maps = _capi.intrinsics(K), torch.empty((H, W, 4), device="cuda"), []
+        for f in (0, 3, 6):
+            d = np.zeros((H, W), np.float32)
+            # a border of zeros in the small image too: beyond it a projection finds no depth in either
+            d[2:h - 2, 2:w - 2] = scenes.render_depth(sc, f)[2:-2, 2:-2]
+            src = torch.from_numpy(d).cuda()
+            backend.integrate_depth_frame_cuda(vol, backend.DepthFrame(K, src.view(-1)), sc.poses[f])
+            _capi.check(_capi.lib().vh_pixel_normals(vol.handle, C.c_void_p(src.data_ptr()), C.c_void_p(nrm.data_ptr()),
+                                                     C.byref(Ki), None), vol.handle)
+            vol.synchronize()
+            maps.append(_bits(nrm.cpu().numpy()[:h, :w]))
+        got = (*O.sort_blocks(*vol.export_blocks()), np.stack(maps))
+        vol.close()
+        want = want or got
+        assert len(got[0]) > 100 and all(np.array_equal(a, b) for a, b in zip(got, want)), (W, H)

@@ -70,6 +70,21 @@ struct Smem {
   float spatial[(2 * kR + 1) * (2 * kR + 1)];
 };
 
+#ifdef VH_FAST_MATH
+// The arithmetic of a tap in the fast-math compile, its multiply-adds written out: with plain operators the compiler picks
+// which product of a sum it fuses, and a pixel's depth would depend on the shape of its tile.
+__device__ __forceinline__ float tap_cosine(f3 cn, const float4& sn) {
+  return clampf(__fmaf_rn(cn.z, sn.z, __fmaf_rn(cn.y, sn.y, __fmul_rn(cn.x, sn.x))), -1.0f, 1.0f);
+}
+// one hardware exponential of the summed exponents: exp(-a) exp(-b) = exp(-(a + b))
+__device__ __forceinline__ float tap_weight(float spatial, float range, bool has_cn, float cosine, const Params& p) {
+  float e = __fmul_rn(range, p.filter_k_range);
+  const float ad = __fsub_rn(1.0f, cosine);
+  if (has_cn) e = __fmaf_rn(__fmul_rn(ad, ad), p.filter_k_angular, e);
+  return __fmul_rn(spatial, __expf(-e));
+}
+#endif
+
 // The taps of radius R around staged pixel (tx, ty), in the reference's order (rows dv outer, columns du
 // inner).  No image-bounds test per tap: the staged tile holds 0 outside the image, which the sd <= 0 test
 // rejects exactly as the reference's bounds test does.
@@ -85,17 +100,16 @@ __device__ __forceinline__ void bilateral_taps(const Smem& S, int tx, int ty, fl
       const float delta = sd - center;
       const float range = delta * delta;
 #ifdef VH_FAST_MATH
-      // one hardware exponential of the summed exponents: exp(-a) exp(-b) = exp(-(a + b))
-      float e = range * p.filter_k_range;
+      float cosine = 0.0f;
       if (has_cn) {
         const float4 sn = S.normal[ty + kR + dv][tx + kR + du];
         if (sn.w == 0.0f) continue;
-        const float cosine = clampf(dot3(cn, mk3(sn.x, sn.y, sn.z)), -1.0f, 1.0f);
+        cosine = tap_cosine(cn, sn);
         if (cosine < p.filter_min_cos) continue;
-        const float ad = 1.0f - cosine;
-        e += ad * ad * p.filter_k_angular;
       }
-      const float w = S.spatial[(dv + kR) * (2 * kR + 1) + (du + kR)] * __expf(-e);
+      const float w = tap_weight(S.spatial[(dv + kR) * (2 * kR + 1) + (du + kR)], range, has_cn, cosine, p);
+      wds = __fmaf_rn(w, sd, wds);
+      ws = __fadd_rn(ws, w);
 #else
       if (adds_zeros(range, p.filter_k_range, p.filter_k_angular)) continue;
       float w = S.spatial[(dv + kR) * (2 * kR + 1) + (du + kR)] * gaussian(range, p.filter_k_range);
@@ -107,9 +121,9 @@ __device__ __forceinline__ void bilateral_taps(const Smem& S, int tx, int ty, fl
         const float ad = 1.0f - cosine;
         w *= gaussian(ad * ad, p.filter_k_angular);
       }
-#endif
       wds += w * sd;
       ws += w;
+#endif
     }
   }
 }
@@ -170,21 +184,19 @@ __device__ __forceinline__ float filter_small_tile(const float* __restrict__ in,
 #endif
     if (in) {
       const float4 sn = S.normal[ty + kR + dv][tx + kR + du];
+      const f3 cn = mk3(cn4.x, cn4.y, cn4.z);
+      const float spatial = S.spatial[(dv + kR) * (2 * kR + 1) + (du + kR)];
 #ifdef VH_FAST_MATH
-      // the fused multiply-adds that the compiler makes of bilateral_taps, written out: the same depth for either tile
-      const float dot = __fmaf_rn(cn4.z, sn.z, __fmaf_rn(cn4.y, sn.y, __fmul_rn(cn4.x, sn.x)));
+      const float cosine = tap_cosine(cn, sn);
 #else
-      const float dot = dot3(mk3(cn4.x, cn4.y, cn4.z), mk3(sn.x, sn.y, sn.z));
-#endif
-      const float cosine = clampf(dot, -1.0f, 1.0f);
+      const float cosine = clampf(dot3(cn, mk3(sn.x, sn.y, sn.z)), -1.0f, 1.0f);
       const float ad = 1.0f - cosine;
+#endif
       if (!has_cn || (sn.w != 0.0f && !(cosine < p.filter_min_cos))) {
 #ifdef VH_FAST_MATH
-        float e = __fmul_rn(range, p.filter_k_range);
-        if (has_cn) e = __fmaf_rn(__fmul_rn(ad, ad), p.filter_k_angular, e);
-        const float w = __fmul_rn(S.spatial[(dv + kR) * (2 * kR + 1) + (du + kR)], __expf(-e));
+        const float w = tap_weight(spatial, range, has_cn, cosine, p);
 #else
-        float w = S.spatial[(dv + kR) * (2 * kR + 1) + (du + kR)] * gaussian(range, p.filter_k_range);
+        float w = spatial * gaussian(range, p.filter_k_range);
         if (has_cn) w *= gaussian(ad * ad, p.filter_k_angular);
 #endif
         t = make_float2(sd, w);
