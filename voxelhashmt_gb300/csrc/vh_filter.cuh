@@ -83,6 +83,12 @@ __device__ __forceinline__ float tap_weight(float spatial, float range, bool has
   if (has_cn) e = __fmaf_rn(__fmul_rn(ad, ad), p.filter_k_angular, e);
   return __fmul_rn(spatial, __expf(-e));
 }
+#else
+// a pixel's taps lie within its threshold of its own depth: finite, if the threshold is (that of an infinite depth is not,
+// or stops every finite tap)
+__device__ __forceinline__ float taps_limit(float thr, const Params& p) {
+  return zeros_limit(thr <= 3.402823466e38f, p.filter_k_angular);
+}
 #endif
 
 // The taps of radius R around staged pixel (tx, ty), in the reference's order (rows dv outer, columns du
@@ -91,6 +97,9 @@ __device__ __forceinline__ float tap_weight(float spatial, float range, bool has
 template <int R>
 __device__ __forceinline__ void bilateral_taps(const Smem& S, int tx, int ty, float center, bool has_cn, f3 cn,
                                                float thr, const Params& p, float& wds, float& ws) {
+#ifndef VH_FAST_MATH
+  const float limit = taps_limit(thr, p);
+#endif
 #pragma unroll
   for (int dv = -R; dv <= R; ++dv) {
 #pragma unroll
@@ -111,7 +120,7 @@ __device__ __forceinline__ void bilateral_taps(const Smem& S, int tx, int ty, fl
       wds = __fmaf_rn(w, sd, wds);
       ws = __fadd_rn(ws, w);
 #else
-      if (adds_zeros(range, p.filter_k_range, p.filter_k_angular)) continue;
+      if (adds_zeros(range, p.filter_k_range, limit)) continue;
       float w = S.spatial[(dv + kR) * (2 * kR + 1) + (du + kR)] * gaussian(range, p.filter_k_range);
       if (has_cn) {
         const float4 sn = S.normal[ty + kR + dv][tx + kR + du];
@@ -170,6 +179,9 @@ __device__ __forceinline__ float filter_small_tile(const float* __restrict__ in,
   const float4 cn4 = S.normal[ty + kR][tx + kR];
   const bool has_cn = cn4.w != 0.0f;
   const float thr = disc_threshold(p, center);
+#ifndef VH_FAST_MATH
+  const float limit = taps_limit(thr, p);
+#endif
   const int side = 2 * p.filter_radius + 1, taps = side * side;
 #pragma unroll 1
   for (int k = tid >> 5; k < taps; k += kSmallThreads / 32) {
@@ -180,7 +192,7 @@ __device__ __forceinline__ float filter_small_tile(const float* __restrict__ in,
     const float range = delta * delta;
     bool in = center > 0.0f && !(sd <= 0.0f) && !(fabsf(delta) > thr);
 #ifndef VH_FAST_MATH
-    in = in && !adds_zeros(range, p.filter_k_range, p.filter_k_angular);
+    in = in && !adds_zeros(range, p.filter_k_range, limit);
 #endif
     if (in) {
       const float4 sn = S.normal[ty + kR + dv][tx + kR + du];

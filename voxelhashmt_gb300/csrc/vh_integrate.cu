@@ -323,6 +323,8 @@ __device__ __forceinline__ bool surface_normal_fast(const float* __restrict__ de
   f3 wsum = cn;
   float ws = 0.0f;
   const bool range_finite = p.normal_k_range <= 3.402823466e38f;  // not for a sigma of 0: the centre's weight is then NaN
+  // a tap that gets as far as its weight has a finite normal, whatever the depths
+  const float limit = zeros_limit(true, p.normal_k_angular);
   // the centre's normal (k = -1), then the nine taps: one copy of the normal's and of the exponential's code
 #pragma unroll 1
   for (int k = -1; k < 9; ++k) {
@@ -337,7 +339,7 @@ __device__ __forceinline__ bool surface_normal_fast(const float* __restrict__ de
       const f3 sp = point(s);
       const float delta = sp.z - cp.z;
       range = delta * delta;
-      if (adds_zeros(range, p.normal_k_range, p.normal_k_angular)) continue;
+      if (adds_zeros(range, p.normal_k_range, limit)) continue;
       // estimateSurfaceNormalBaseCamera on the samples, toward the camera
       const f3 cr = cross3(sub3(point(b), point(a)), sub3(point(s + 1), point(s - 1)));
       const float len = norm3(cr);
