@@ -638,18 +638,46 @@ __device__ __forceinline__ bool integrate_bin16(const Params& p, const Volume& V
   return true;
 }
 
+#ifdef VH_FAST_MATH
+// The fast-math compile leaves to the compiler which product of a sum is fused and what becomes of a quotient, and it
+// chooses anew in each kernel.  What two kernels have to agree on is written out, in the form that it chose for the
+// fused update.
+__device__ __forceinline__ float rcp_approx(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float row_dot(float a, float b, float c, f3 p) {
+  return __fmaf_rn(c, p.z, __fmaf_rn(a, p.x, __fmul_rn(b, p.y)));
+}
+#endif
+
 // First part of integrateActiveBlocksKernel for one voxel (:849-877): voxel centre, projection, bilinear
 // depth, truncation test.  Returns false when the reference returns before touching the voxel.
+//
+// The plain form's update projects a listed voxel again and takes it for inside the image, its centre sample for valid and its
+// kind (shared samples or literal) for the right one.  A last bit of difference to the classify pass's projection, at the
+// image's border or beside a pixel without depth, left the update without a centre sample.
 __device__ __forceinline__ bool voxel_projection(const Params& p, const int4& bk, int li, f3& pc, float& u, float& v) {
   const int lx = li & 7, ly = (li >> 3) & 7, lz = li >> 6;
   const f3 pw = mk3((static_cast<float>(bk.x * kBlockSide + lx) + 0.5f) * p.voxel_size,
                     (static_cast<float>(bk.y * kBlockSide + ly) + 0.5f) * p.voxel_size,
                     (static_cast<float>(bk.z * kBlockSide + lz) + 0.5f) * p.voxel_size);
+#ifdef VH_FAST_MATH
+  const Mat34& T = p.T_cw;
+  pc = mk3(__fadd_rn(row_dot(T.r[0], T.r[1], T.r[2], pw), T.t[0]), __fadd_rn(row_dot(T.r[3], T.r[4], T.r[5], pw), T.t[1]),
+           __fadd_rn(row_dot(T.r[6], T.r[7], T.r[8], pw), T.t[2]));
+  if (pc.z <= 1e-6f) return false;
+  const float inv_z = rcp_approx(pc.z);
+  u = __fmaf_rn(__fmul_rn(p.fx, pc.x), inv_z, p.cx);
+  v = __fmaf_rn(__fmul_rn(p.fy, pc.y), inv_z, p.cy);
+#else
   pc = xform_point(p.T_cw, pw);
   if (pc.z <= 0.0f) return false;
   if (pc.z <= 1e-6f) return false;
   u = p.fx * pc.x / pc.z + p.cx;
   v = p.fy * pc.y / pc.z + p.cy;
+#endif
   return u >= 0.0f && u <= static_cast<float>(p.width - 1) && v >= 0.0f && v <= static_cast<float>(p.height - 1);
 }
 
