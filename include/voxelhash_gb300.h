@@ -106,9 +106,9 @@ typedef struct vh_algorithm {
   int32_t normal_mode;
   /* 1 (default): with normal_mode 1, the first frames cycle the layer-update kernel through its launch shapes
    * (threads per CTA x minimum resident CTAs per SM x voxel slots a thread tests per pass), time each with CUDA
-   * events and keep the fastest (with fast_math 0 the results do not depend on the shape; with fast_math 1 about one
-   * word in a hundred thousand differs in its last bits, the compiler taking the reciprocal root for a quotient
-   * in some shapes); 0: the shape launch_variant. */
+   * events and keep the fastest (the results do not depend on the shape, except that with fast_math 1 and FP16 storage
+   * about one word in a hundred thousand differs in its last bits, where the compiler takes the reciprocal root for
+   * a quotient in some shapes); 0: the shape launch_variant. */
   int32_t autotune;
   int32_t launch_variant; /* the layer-update launch shape used without autotuning (0..9, default 0) */
   /* 0 (default): the reference's bilateral depth filter; 1: the learned depth denoiser set with

@@ -493,6 +493,40 @@ def test_fast_math_normals_per_voxel_are_reproducible(env, alloc, fp16):
     assert len(want[0]) > 10000
 
 
+@pytest.mark.parametrize("scene", ["room", "object"])
+def test_fast_math_records_do_not_depend_on_the_launch(env, scene):
+    """With FP32 bins the fast-math compile fuses the same words in each of the update's ten launch shapes, and as a batch of one
+    (one launch per kernel, one graph, one persistent launch)."""
+    backend, O = env
+    from voxelhashmt_gb300 import _capi, denoiser, scenes
+    if scene == "room":
+        sc = scenes.room_scene(1, frames=64)
+        sc.voxel_size, sc.truncation, sc.poses = 0.005, 0.02, sc.poses[1:5]
+    else:
+        sc = scenes.object_scan_scene(3, frames=24, resolution=(160, 120), voxel_size=0.008)
+        sc.truncation = 4.0 * sc.voxel_size
+    frames, want = denoiser.render_frames(sc, torch), None
+    for launch in [*range(10), False, True, "persistent"]:
+        single = not isinstance(launch, (bool, str))
+        vol = backend.VoxelHashTSDF(sc.voxel_size, sc.truncation, hash_buckets=1 << 18, max_blocks=16384,
+                                    algorithm=_capi.default_algorithm(allocation_mode=1, normal_mode=1, fast_math=1, autotune=0,
+                                                                      launch_variant=launch if single else 0))
+        batch = None if single else backend.VolumeBatch([vol], launch)
+        for d, pose in zip(frames, sc.poses):
+            if single:
+                backend.integrate_depth_frame_cuda(vol, backend.DepthFrame(sc.intrinsics, d.view(-1)), pose, synchronize=False)
+            else:
+                batch.integrate([d], [sc.intrinsics], [pose], 1)
+        vol.synchronize()
+        got = _device_blocks(vol)
+        if batch:
+            batch.close()
+        vol.close()
+        want = want or got
+        assert all(torch.equal(a, b) for a, b in zip(got, want)), launch
+    assert len(want[0]) > 500
+
+
 def _device_blocks(vol):
     """(keys, voxel words) of a volume in the order of the keys, on the device."""
     from voxelhashmt_gb300 import _capi

@@ -397,6 +397,22 @@ __device__ __forceinline__ bool shifts_exact(float u, float v) {
          floorf(up1 + 1.0f) == floorf(u) + 2.0f && floorf(vp1 + 1.0f) == floorf(v) + 2.0f;
 }
 
+#ifdef VH_FAST_MATH
+// The fast-math compile leaves to the compiler which product of a sum is fused and what becomes of a quotient, and it
+// chooses anew in each kernel and launch shape.  What several of them have to agree on is written out: the projection of a
+// voxel (classify and update), in the form that it chose for the fused update, and the length of a record's normal
+// (the launch shapes of the fused update and the batch), by the reciprocal root that it took in four of the ten shapes and in
+// the batch.
+__device__ __forceinline__ float rcp_approx(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float row_dot(float a, float b, float c, f3 p) {
+  return __fmaf_rn(c, p.z, __fmaf_rn(a, p.x, __fmul_rn(b, p.y)));
+}
+#endif
+
 // computeObservationWeightGpu (cuda_tsdf_integrator.cu:429-450)
 __device__ __forceinline__ float observation_weight(const Params& p, float depth, float sd, float view) {
   if (depth <= 0.0f || p.truncation <= 1e-6f) return 0.0f;
@@ -463,7 +479,12 @@ __device__ __forceinline__ f3 unpack_normal(uint32_t packed) {
     n.x = fx;
     n.y = fy;
   }
+#ifdef VH_FAST_MATH
+  const float inv = rsqrtf(row_dot(n.x, n.y, n.z, n));  // of a length between 0.57 and 1
+  return mk3(__fmul_rn(n.x, inv), __fmul_rn(n.y, inv), __fmul_rn(n.z, inv));
+#else
   return normalize3(n);
+#endif
 }
 
 __device__ __forceinline__ bool layer_valid(const float4& l) { return l.x > 0.0f; }
@@ -637,20 +658,6 @@ __device__ __forceinline__ bool integrate_bin16(const Params& p, const Volume& V
   B = make_uint4(p16[2], w16[0] ? nk[0] : 0U, w16[1] ? nk[1] : 0U, w16[2] ? nk[2] : 0U);
   return true;
 }
-
-#ifdef VH_FAST_MATH
-// The fast-math compile leaves to the compiler which product of a sum is fused and what becomes of a quotient, and it
-// chooses anew in each kernel.  What two kernels have to agree on is written out, in the form that it chose for the
-// fused update.
-__device__ __forceinline__ float rcp_approx(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-__device__ __forceinline__ float row_dot(float a, float b, float c, f3 p) {
-  return __fmaf_rn(c, p.z, __fmaf_rn(a, p.x, __fmul_rn(b, p.y)));
-}
-#endif
 
 // First part of integrateActiveBlocksKernel for one voxel (:849-877): voxel centre, projection, bilinear
 // depth, truncation test.  Returns false when the reference returns before touching the voxel.
