@@ -47,10 +47,10 @@ PEAKS_FALLBACK = {"hbm_gbs": 6800.0}
 # bytes per active voxel, written bytes per updated voxel), scaled by the active and updated voxels of a launch
 # (plain: update_kernel_room640.md, one launch over 6.55 M active voxels, read + write per active voxel;
 # opt-in form: fused_update_room640.md, one launch over 3.16 M active and 2.86 M updated voxels).
-UPDATE_TRAFFIC_BYTES = {"plain": ((536.541e6 + 265.530e6) / 6.549e6, 0.0),
+UPDATE_TRAFFIC_BYTES = {"plain": ((536.231e6 + 263.150e6) / 6.549e6, 0.0),
                         "chosen": (189.529e6 / 3.163e6, 58.035e6 / 2.860e6)}
 # warp instructions per active voxel of the layer-update kernel (smsp__inst_executed.sum of the same captures)
-UPDATE_WARP_INSTRUCTIONS = {"plain": 1336.314e6 / 6.549e6, "chosen": 111.551e6 / 3.163e6}
+UPDATE_WARP_INSTRUCTIONS = {"plain": 1329.895e6 / 6.549e6, "chosen": 111.551e6 / 3.163e6}
 
 
 def parse():
@@ -591,14 +591,16 @@ def run_gb300(args):
             cpu = {"value": None, "unit": "Mpix/s", "cores": 0, "kind": "port", "sample": "failed: %s" % e}
 
     def mc_roofline(r, name):
-        # the survey's algorithmic bytes of one extraction: per block one read of its 512 voxels' bins in all 6
-        # directions, the one-voxel halo (217 voxels x 6 directions), and 36 B per emitted triangle
+        # nominal bytes of one extraction: per block one read of its 512 voxels' bins in all 6 directions, the one-voxel
+        # halo (217 voxels x 6 directions), and 36 B per emitted triangle.  The kernels read fewer (observed voxels' bins in
+        # the directions that hold any, then the corner bins of marked cells) and are bound by instruction issue.
         bin_b = BIN_BYTES[FORMS[name][1]]
         nbytes = r["nblocks"] * (512 + 217) * 6 * bin_b + 36 * r["triangles"]
         ach = nbytes / (r["mc_ms"] / 1000.0) / 1e9
-        return {"kernels": "near_kernel + cells_kernel (count) + scans + cells_kernel (emit) (one full extraction)", "bound": "hbm",
+        return {"kernels": "near_kernel + cells_kernel (count) + scans + cells_kernel (emit) (one full extraction)", "bound": "issue",
                 "achieved": round(ach, 2), "peak": pk["hbm_gbs"], "unit": "GB/s", "frac": round(ach / pk["hbm_gbs"], 5),
-                "algorithmic_bytes": int(nbytes), "ms": round(r["mc_ms"], 3)}
+                "nominal_bytes": int(nbytes), "ms": round(r["mc_ms"], 3),
+                "note": "every bin of every block and of its halo, most of which the kernels never read: not traffic"}
 
     def summary(r, name):
         return {"form": FORM_NOTE[name], "integrated_mpix_per_s": round(r["value"], 3),

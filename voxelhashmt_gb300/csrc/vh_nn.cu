@@ -565,8 +565,9 @@ cudaError_t launch_pack_w32(const float* w, __nv_bfloat16* out, int transpose_fl
 // read.  The gradient row is staged the same way as the B operand, [pixel group][output channel][8 pixels].  A
 // thread loads a channel pair over 10 (8) pixels as 32-bit words and writes the transposed 16-byte rows with
 // byte permutes; the loads of a row are issued a row ahead, so they are in flight while the row before it is
-// staged and multiplied (a batch of 16 640x480 frames: 374 -> 287 us, shared-memory traffic now the largest part).  Rows live in rings (three input rows, two gradient rows); thread 0 issues an output
-// row's 12 MMAs (3 tap rows x 4 k-steps of 16 pixels) and commits them to an mbarrier, and a ring slot is
+// staged and multiplied (a batch of 16 640x480 frames: 374 -> 330 us on average, 372 and 287 for the two layers; the
+// rows' barriers and the loads' latency are the largest stalls).  Rows live in rings (three input rows, two
+// gradient rows); thread 0 issues an output row's 12 MMAs (3 tap rows x 4 k-steps of 16 pixels) and commits them to an mbarrier, and a ring slot is
 // rewritten only after the MMAs that read it have completed.  Four CTAs per SM (their tensor memory fills the
 // SM's 512 columns).  Waits are bounded as in conv32_tc_kernel; a timeout is agreed on by every thread
 // (__syncthreads_and) before the CTA leaves its loop.

@@ -23,7 +23,7 @@
 // neighbourhood moves one voxel along an axis half of the lanes keep theirs: a voxel's plane (its choice depends on
 // the ray's direction alone, not on the sample) stays in registers until its lane moves on.  A voxel without an
 // observed layer is known from its bit of the observed-voxel mask, without reading bins.  The same view takes
-// 6.3 ms; the kernel is bound by instruction issue (53 % of the slots, 20 of 32 threads active).  Measured and not
+// 6.3 ms; the kernel is bound by instruction issue (75 % of the slots, 21 of 32 threads active).  Measured and not
 // kept: one lane per ray through unallocated space and eight through blocks, handing over inside a warp
 // (12-21 ms) or inside a CTA with a list of rays (6.7-25 ms): rays that run through blocks out of step execute both
 // parts of the loop.
